@@ -38,6 +38,11 @@ struct efsi_ib_search_plan {
   unsigned long long* host_total = nullptr;  // and its pinned readback
   int32_t* claim = nullptr;  // per fluid cell: relocation claims, then region writers
   int64_t claim_cap = 0;
+  float4* rec = nullptr;  // per item: kRecQuads quads of precomputed geometry
+  int64_t rec_cap = 0;
+  uint32_t* far_nodes = nullptr;  // nodes whose far classification is still open, and their count
+  int64_t far_cap = 0;
+  unsigned* far_count = nullptr;
 };
 
 namespace efsi {
@@ -133,6 +138,9 @@ struct SearchArgs {
   int nb[3];
   const int32_t* offset;   // null: every node visits every item
   const int32_t* entries;
+  const float4* rec;       // per item: kRecQuads quads (k_ibs_records)
+  uint32_t* far_nodes;     // nodes left to k_ibs_far, and their count
+  unsigned* far_count;
   // per-node fields (hibm_mpm.py:5418-5436) and the four report counts
   int32_t* kind;
   int32_t* nearest;
@@ -174,24 +182,68 @@ __device__ __forceinline__ F3 oriented_normal(const SearchArgs& A, F3 fn, int ia
   return normal;
 }
 
-// Distance and signed distance of node p to item t (hibm_mpm.py:5900-5920 /
-// 5967-5970); false for a degenerate triangle, which the node skips.
-__device__ bool item_eval(const SearchArgs& A, int t, F3 p, float& distance, float& sdist) {
-  if (A.tri_count > 0) {
-    int ia, ib, ic;
-    if (!tri_indices(A, t, ia, ib, ic)) return false;
-    F3 closest, fn;
-    if (!closest_point(p, ld3(A.mx, ia), ld3(A.mx, ib), ld3(A.mx, ic), closest, fn)) return false;
-    const F3 normal = oriented_normal(A, fn, ia, ib, ic);
-    const F3 off = sub(p, closest);
-    distance = norm(off);
-    sdist = dot(off, normal);
-    return true;
+// Geometry of an item that no node changes, formed once per search by
+// k_ibs_records (a triangle's corners, its oriented unit normal; a marker's
+// position and normal), and what bounds its distances from below:
+//   q0 = (a, reach)   reach: the largest distance of the item's points from a
+//   q1 = (n, slack)   |s - dot(p - a, n)| <= slack + kSlackP |p|_1
+//   q2 = (b, -), q3 = (c, -)
+// The items of one warp's lanes are read as whole quads.
+constexpr int kRecQuads = 4;
+constexpr float kSlack = 2.0e-5f;  // about 300 f32 units in the last place
+
+__device__ __forceinline__ F3 xyz(float4 q) { return f3(q.x, q.y, q.z); }
+__device__ __forceinline__ float abs1(F3 v) { return fabsf(v.x) + fabsf(v.y) + fabsf(v.z); }
+
+__global__ void k_ibs_records(SearchArgs A, float4* rec) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= items(A)) return;
+  float4* r = rec + (int64_t)kRecQuads * t;
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  r[2] = r[3] = zero;
+  if (A.tri_count == 0) {
+    const F3 x = ld3(A.mx, t), n = ld3(A.mn, t);
+    r[0] = make_float4(x.x, x.y, x.z, kSlack * abs1(x));
+    r[1] = make_float4(n.x, n.y, n.z, kSlack * abs1(x));
+    return;
   }
-  const F3 off = sub(p, ld3(A.mx, t));
+  int ia, ib, ic;
+  F3 closest, fn;
+  const float never = __int_as_float(0xff800000);  // reach and slack of a degenerate item: no test asks for it
+  r[0] = r[1] = make_float4(0.0f, 0.0f, 0.0f, never);
+  if (!tri_indices(A, t, ia, ib, ic)) return;
+  const F3 a = ld3(A.mx, ia), b = ld3(A.mx, ib), c = ld3(A.mx, ic);
+  if (!closest_point(a, a, b, c, closest, fn)) return;
+  const F3 n = oriented_normal(A, fn, ia, ib, ic);
+  const F3 ab = sub(b, a), ac = sub(c, a), bc = sub(c, b);
+  const float lab = norm(ab), lac = norm(ac), lbc = norm(bc);
+  const float coords = kSlack * (abs1(a) + abs1(b) + abs1(c));
+  // In exact arithmetic p - closest and p - a have the same component along
+  // the normal.  In f32 they differ by the rounding of the coordinates and by
+  // how far the rounded edges leave the plane of the rounded normal.  A
+  // triangle whose angles leave too little of the cross product, or whose
+  // edges are too short for the barycentric sums of a distant node, gets no
+  // bound (infinite slack): it is always evaluated.
+  float slack = 4.0f * (fabsf(dot(ab, n)) + fabsf(dot(ac, n))) + coords;
+  const float shortest = fminf(lab, fminf(lac, lbc));
+  if (!(norm(cross(ab, ac)) > 1.0e-3f * lab * lac) || !(shortest > 1.0e-4f * (abs1(a) + abs1(b) + abs1(c))))
+    slack = __int_as_float(0x7f800000);
+  r[0] = make_float4(a.x, a.y, a.z, fmaxf(lab, lac) * 1.0001f + coords);
+  r[1] = make_float4(n.x, n.y, n.z, slack);
+  r[2] = make_float4(b.x, b.y, b.z, 0.0f);
+  r[3] = make_float4(c.x, c.y, c.z, 0.0f);
+}
+
+// Distance and signed distance of node p to item t (hibm_mpm.py:5900-5920 /
+// 5967-5970), from its record; the item must not be degenerate.
+__device__ void item_eval(const SearchArgs& A, int t, F3 p, float& distance, float& sdist) {
+  const float4* r = A.rec + (int64_t)kRecQuads * t;
+  const F3 a = xyz(__ldg(r)), n = xyz(__ldg(r + 1));
+  F3 closest = a, fn;
+  if (A.tri_count > 0) closest_point(p, a, xyz(__ldg(r + 2)), xyz(__ldg(r + 3)), closest, fn);
+  const F3 off = sub(p, closest);
   distance = norm(off);
-  sdist = dot(off, ld3(A.mn, t));
-  return true;
+  sdist = dot(off, n);
 }
 
 __device__ __forceinline__ float clamp01(float v) { return fminf(fmaxf(v, 0.0f), 1.0f); }
@@ -396,6 +448,23 @@ __global__ void __launch_bounds__(kScanThreads) k_ibs_offsets(const int32_t* cou
   if (base <= n - 1 && n - 1 < base + kScanPer) offset[n] = run;  // the entry total
 }
 
+// A far node stays "none" as soon as one item sees it outside, whichever it
+// is: a spread of kFarSamples items settles nearly all of them.
+constexpr int kFarSamples = 64;
+
+__device__ bool far_open(const SearchArgs& A, F3 p, float slack_p) {
+  const int n = items(A);
+  if (n == 0) return false;  // no item: "none"
+  const int m = min(n, kFarSamples), stride = n / m;
+  for (int q = 0; q < m; ++q) {
+    const int t = (int)((int64_t)n * q / m) + (q * 37) % stride;
+    const float4 q0 = __ldg(A.rec + (int64_t)kRecQuads * t), q1 = __ldg(A.rec + (int64_t)kRecQuads * t + 1);
+    const float s = dot(sub(p, xyz(q0)), xyz(q1));
+    if (q1.w >= 0.0f && s > A.tol + (q1.w + slack_p)) return false;
+  }
+  return true;
+}
+
 // One thread per node (hibm_mpm.py:5837-6068 / 5603-5835).
 __global__ void __launch_bounds__(256) k_ibs_search(SearchArgs A) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -414,10 +483,17 @@ __global__ void __launch_bounds__(256) k_ibs_search(SearchArgs A) {
     hi_e = __ldg(A.offset + b + 1);
     list = A.entries;
   }
+  const float slack_p = kSlack * abs1(p);
   for (int e = lo_e; e < hi_e; ++e) {
     const int t = list != nullptr ? __ldg(list + e) : e;
+    // only items closer than the radius matter here: the rest are told apart
+    // by their corner a and reach
+    const float4 q0 = __ldg(A.rec + (int64_t)kRecQuads * t);
+    const F3 oa = sub(p, xyz(q0));
+    const float lim = A.radius + q0.w + slack_p;
+    if (!(lim > 0.0f) || dot(oa, oa) > lim * lim) continue;
     float d, s;
-    if (!item_eval(A, t, p, d, s)) continue;
+    item_eval(A, t, p, d, s);
     if (d < A.radius) {
       if (s > A.tol) {
         external_seen = true;
@@ -448,28 +524,9 @@ __global__ void __launch_bounds__(256) k_ibs_search(SearchArgs A) {
       kind = kNodeInternal;
       atomicAdd(A.report + 2, 1);
     }
-  } else if (A.classify_far) {
-    Best global;
-    bool global_external_seen = false;
-    const int nitems = items(A);
-    for (int t = 0; t < nitems; ++t) {
-      float d, s;
-      if (!item_eval(A, t, p, d, s)) continue;
-      if (s > A.tol) {
-        global_external_seen = true;  // the node stays "none"
-        break;
-      }
-      global.offer(d, t);
-    }
-    if (!global_external_seen && global.t >= 0) {
-      kind = kNodeInternal;
-      F3 normal;
-      item_detail(A, global.t, p, marker, boundary, normal, ix, w);
-      float dsel;
-      item_eval(A, global.t, p, dsel, sd);
-      interior = add(boundary, scale(normal, A.probe));
-      atomicAdd(A.report + 2, 1);
-    }
+  } else if (A.classify_far && far_open(A, p, slack_p)) {
+    // the node may be internal: k_ibs_far looks at every item
+    A.far_nodes[atomicAdd(A.far_count, 1u)] = (uint32_t)c;
   }
   A.kind[c] = kind;
   A.nearest[c] = marker;
@@ -479,6 +536,99 @@ __global__ void __launch_bounds__(256) k_ibs_search(SearchArgs A) {
   for (int q = 0; q < 3; ++q) {
     A.pidx[3 * c + q] = ix[q];
     A.pw[3 * c + q] = w[q];
+  }
+}
+
+// The far nodes k_ibs_search left open (hibm_mpm.py:5937-6010: internal when no
+// item at all sees the node outside, with the nearest of all items).  Every
+// item has to be looked at for every node, so what counts is the cost of a
+// look: a warp holds kFarNodes nodes, its lanes take the items of a tile that
+// the block has staged in shared memory (two quads an item), and an item is
+// evaluated in full only when its bound cannot tell that it is inside and
+// farther than the best so far.  One thread per node over all items took
+// 33.8 of the boundary rows' 34.2 ms on a 96 x 96 x 128 grid with 9,024
+// triangles: every evaluation formed the triangle's normal again, and the
+// internal nodes kept a few warps per SM busy with one serial chain each.  The
+// whole of the rows now takes 5.9 ms; the bound tests' issue slots are what is
+// left of it.
+constexpr int kFarNodes = 4, kFarWarps = 8, kFarTile = 256;
+
+__global__ void __launch_bounds__(kFarWarps * 32) k_ibs_far(SearchArgs A) {
+  __shared__ float4 tile[2][kFarTile];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t count = *A.far_count;
+  const int n = items(A);
+  constexpr int kPerBlock = kFarNodes * kFarWarps;
+  for (int64_t base = (int64_t)blockIdx.x * kPerBlock; base < count; base += (int64_t)gridDim.x * kPerBlock) {
+    F3 p[kFarNodes];
+    float slack_p[kFarNodes];
+    Best best[kFarNodes];
+    unsigned open = 0;  // nodes of this warp that no item has seen outside
+#pragma unroll
+    for (int q = 0; q < kFarNodes; ++q) {
+      const int64_t e = base + warp * kFarNodes + q;
+      const int64_t c = A.far_nodes[e < count ? e : count - 1];
+      p[q] = node_position(A, (int)(c / ((int64_t)A.ny * A.nz)), (int)((c / A.nz) % A.ny), (int)(c % A.nz));
+      slack_p[q] = kSlack * abs1(p[q]);
+      if (e < count) open |= 1u << q;
+    }
+    for (int t0 = 0; t0 < n; t0 += kFarTile) {
+      // also the barrier between the last tile's reads and this one's writes
+      if (!__syncthreads_or(open != 0)) break;
+      const int tn = min(kFarTile, n - t0);
+      for (int q = threadIdx.x; q < 2 * tn; q += blockDim.x)
+        tile[q & 1][q >> 1] = __ldg(A.rec + (int64_t)kRecQuads * (t0 + (q >> 1)) + (q & 1));
+      __syncthreads();
+      if (open == 0) continue;
+      for (int u = lane; u < tn; u += 32) {
+        const float4 q0 = tile[0][u], q1 = tile[1][u];
+#pragma unroll
+        for (int q = 0; q < kFarNodes; ++q) {
+          const F3 off = sub(p[q], xyz(q0));
+          const float s = dot(off, xyz(q1)), lim = best[q].d + q0.w + slack_p[q];
+          const bool maybe_outside = s > A.tol - (q1.w + slack_p[q]);
+          const bool maybe_nearest = lim > 0.0f && dot(off, off) <= lim * lim;
+          if ((open >> q & 1u) && (maybe_outside || maybe_nearest)) {
+            float d, se;
+            item_eval(A, t0 + u, p[q], d, se);
+            if (se > A.tol)
+              open &= ~(1u << q);
+            else
+              best[q].offer(d, t0 + u);
+          }
+        }
+      }
+      open = __reduce_and_sync(0xffffffffu, open);
+    }
+    __syncthreads();  // the tile is staged again for the next nodes
+#pragma unroll
+    for (int q = 0; q < kFarNodes; ++q) {
+      // the lanes' lexicographic minima of (distance, index)
+      Best b = best[q];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float d = __shfl_xor_sync(0xffffffffu, b.d, o);
+        const int t = __shfl_xor_sync(0xffffffffu, b.t, o);
+        if (t >= 0) b.offer(d, t);
+      }
+      if (!(open >> q & 1u) || b.t < 0 || lane != 0) continue;
+      int marker, ix[3];
+      float w[3], d, sd;
+      F3 boundary, normal;
+      item_detail(A, b.t, p[q], marker, boundary, normal, ix, w);
+      item_eval(A, b.t, p[q], d, sd);
+      const int64_t c = A.far_nodes[base + warp * kFarNodes + q];
+      A.kind[c] = kNodeInternal;
+      A.nearest[c] = marker;
+      A.sd[c] = sd;
+      st3(A.bp, c, boundary);
+      st3(A.ip, c, add(boundary, scale(normal, A.probe)));
+      for (int a = 0; a < 3; ++a) {
+        A.pidx[3 * c + a] = ix[a];
+        A.pw[3 * c + a] = w[a];
+      }
+      atomicAdd(A.report + 2, 1);
+    }
   }
 }
 
@@ -942,8 +1092,10 @@ int efsi_ib_search_plan_create(efsi_ib_search_plan** out) {
   EFSI_ARG_CHECK(out != nullptr, "null plan pointer");
   efsi_ib_search_plan* P = new efsi_ib_search_plan();
   if (cudaMalloc(&P->total, sizeof(unsigned long long)) != cudaSuccess ||
+      cudaMalloc(&P->far_count, sizeof(unsigned)) != cudaSuccess ||
       cudaMallocHost(&P->host_total, sizeof(unsigned long long)) != cudaSuccess) {
     cudaFree(P->total);
+    cudaFree(P->far_count);
     delete P;
     set_error("cudaMallocHost failed for the node-search readback");
     return EFSI_ERR_CUDA;
@@ -960,6 +1112,9 @@ int efsi_ib_search_plan_destroy(efsi_ib_search_plan* P) {
   cudaFree(P->tile_sums);
   cudaFree(P->entries);
   cudaFree(P->claim);
+  cudaFree(P->rec);
+  cudaFree(P->far_nodes);
+  cudaFree(P->far_count);
   cudaFree(P->total);
   cudaFreeHost(P->host_total);
   delete P;
@@ -1051,7 +1206,18 @@ int efsi_ib_node_search(efsi_ib_search_plan* P, const efsi_ib_search_params* prm
   const int nitems = prm->triangle_count > 0 ? prm->triangle_count : prm->marker_count;
   A.offset = nullptr;
   A.entries = nullptr;
+  EFSI_TRY(grow(P->rec, P->rec_cap, (int64_t)kRecQuads * std::max(nitems, 1)));
+  A.rec = P->rec;
+  if (A.classify_far) {
+    // 32-bit node indices: 2^32 nodes' fields would not fit the device
+    EFSI_ARG_CHECK(A.n < (int64_t)1 << 32, "too many nodes");
+    EFSI_TRY(grow(P->far_nodes, P->far_cap, A.n));
+    A.far_nodes = P->far_nodes;
+    A.far_count = P->far_count;
+    EFSI_CUDA_CHECK(cudaMemsetAsync(P->far_count, 0, sizeof(unsigned), s));
+  }
   if (nitems > 0) {
+    EFSI_COUNTED k_ibs_records<<<(unsigned)((nitems + 255) / 256), 256, 0, s>>>(A, P->rec);
     const int64_t tiles = (nbins + kScanTile - 1) / kScanTile;
     if (nbins > P->bin_cap) {
       cudaFree(P->count);
@@ -1090,6 +1256,7 @@ int efsi_ib_node_search(efsi_ib_search_plan* P, const efsi_ib_search_params* prm
     }
   }
   EFSI_COUNTED k_ibs_search<<<(unsigned)((A.n + 255) / 256), 256, 0, s>>>(A);
+  if (A.classify_far && nitems > 0) EFSI_COUNTED k_ibs_far<<<4 * 148, kFarWarps * 32, 0, s>>>(A);
   EFSI_LAUNCH_CHECK();
   return EFSI_OK;
 }

@@ -1,0 +1,82 @@
+"""Kernels at the sizes where their tiles, remainders and selection rules can
+go wrong, against the CPU oracle or a plain float64 restatement."""
+
+import numpy as np
+import pytest
+
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+# ---------------------------------------------------------------------------
+# far nodes of the immersed-boundary search
+# ---------------------------------------------------------------------------
+
+
+def _closed_surface(bands, slivers):
+    """A UV sphere's markers and triangles; with `slivers`, also triangles
+    that the distance bound must not judge: nearly collinear ones, tiny ones
+    and degenerate ones, on and inside the sphere."""
+    from easyfsi_b200.geometry import UvSphereResolution, make_uv_sphere
+
+    mesh = make_uv_sphere(UvSphereResolution(bands, 2 * bands), 0.33)
+    x = mesh.vertices + 0.5
+    n = mesh.vertices / 0.33
+    tri = [tuple(int(v) for v in f) for f in mesh.faces]
+    if slivers:
+        rng = np.random.default_rng(bands)
+        base = len(x)
+        extra, normals = [], []
+        for q in range(12):
+            u = rng.normal(size=3)
+            u /= np.linalg.norm(u)
+            v = np.cross(u, rng.normal(size=3))
+            v /= np.linalg.norm(v)
+            c = 0.5 + 0.33 * u
+            size = 0.05 if q % 3 == 0 else 1.0e-4
+            off = np.cross(u, v) * size * (1.0e-4 if q % 2 else 0.5)
+            extra += [c, c + size * v, c + 0.5 * size * v + off]
+            normals += [u] * 3
+            tri.append((base + 3 * q, base + 3 * q + 1, base + 3 * q + 2))
+        tri += [(base, base, base + 1), (base, base + 1, base)]  # degenerate
+        x = np.concatenate([x, np.asarray(extra)])
+        n = np.concatenate([n, np.asarray(normals)])
+    return x.astype(np.float32), n.astype(np.float32), np.asarray(tri, np.int32)
+
+
+@pytest.mark.parametrize("bands,slivers,triangles,nodes", [
+    (3, False, True, (9, 11, 13)),     # fewer triangles than lanes and samples
+    (6, True, True, (17, 9, 21)),      # one tile of items, ill-shaped triangles
+    (12, False, False, (16, 16, 19)),  # markers without triangles
+    (16, True, True, (20, 23, 31)),    # several tiles with a remainder
+])
+def test_far_nodes_match_the_all_pairs_oracle(bands, slivers, triangles, nodes):
+    """Kinds, nearest markers and projection indices identical to the oracle's
+    loop over every item; distances and points within 1e-6 (the same f32
+    expressions)."""
+    from easyfsi_b200.hibm_mpm import HibmMpmIbNodeSearch, HibmMpmSurfaceMarkers
+
+    x, n, tri = _closed_surface(bands, slivers)
+    mk = HibmMpmSurfaceMarkers(marker_capacity=len(x), projection_triangle_capacity=len(tri))
+    mk.load_markers(positions_m=x.tolist(), velocities_mps=np.zeros_like(x).tolist(), normals=n.tolist(),
+                    areas_m2=[1.0] * len(x), region_ids=[1] * len(x))
+    if triangles:
+        mk.set_projection_triangles(tri.tolist())
+    search = HibmMpmIbNodeSearch(grid_nodes=nodes, bounds_min_m=(0.0, 0.0, 0.0), bounds_max_m=(1.0, 1.0, 1.0),
+                                 marker_capacity=len(x))
+    rep = search.search_and_classify(mk, search_radius_m=0.03, interior_probe_distance_m=0.02,
+                                     classify_far_internal_nodes=True)
+    ref = orc.ib_node_search(grid_nodes=nodes, markers_x=mk.x_gamma_m.to_numpy(), markers_n=mk.n_gamma.to_numpy(),
+                             triangles=tri if triangles else None, search_radius=0.03, interior_probe_distance=0.02,
+                             sign_tolerance=search._default_sign_tolerance_m(), classify_far=True,
+                             bounds_min=(0.0, 0.0, 0.0), spacing=search.spacing_m)
+    assert rep.__dict__ == ref["report"]
+    assert rep.internal_node_count > 0
+    np.testing.assert_array_equal(search.node_kind_code.to_numpy(), ref["kind"])
+    np.testing.assert_array_equal(search.nearest_marker.to_numpy(), ref["nearest_marker"])
+    np.testing.assert_array_equal(search.node_projection_marker_indices.to_numpy(), ref["projection_indices"])
+    for got, key in ((search.node_signed_distance_m, "signed_distance"), (search.node_boundary_point_m, "boundary_point"),
+                     (search.node_interior_fluid_point_m, "interior_point"),
+                     (search.node_projection_marker_weights, "projection_weights")):
+        np.testing.assert_allclose(got.to_numpy(), ref[key], rtol=0.0, atol=1e-6, err_msg=key)

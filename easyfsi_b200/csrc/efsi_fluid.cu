@@ -259,52 +259,192 @@ __device__ __forceinline__ void sample_prev(const LevelDev& L, const float* __re
   }
 }
 
-// fluid.py:2447-2513 _predict_kernel.
-__global__ void __launch_bounds__(256) k_predict(LevelDev L, efsi_grid_axes A, const float* __restrict__ vp,
-                                                 float dt, float nu, int rk2, float* __restrict__ vel) {
-  EFSI_CELL(L)
-  const unsigned m = __ldg(L.mask + c);
-  if (m & M_SOLID) {
-    vel[3 * c] = vel[3 * c + 1] = vel[3 * c + 2] = 0.0f;
+// x / w with r = 1 / w rounded to nearest: the product x r, corrected by its
+// exact remainder (Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", 1990), rounds as the quotient does while
+// nothing underflows; a non-finite remainder (x infinite or NaN, or the
+// quotient overflowing) leaves the product.  Three instructions and a select
+// instead of the full division, for the divisors a thread meets many times.
+__device__ __forceinline__ float div_by(float x, float w, float r) {
+  const float q = __fmul_rn(x, r);
+  const float e = __fmaf_rn(-q, w, x);
+  return fabsf(e) <= 3.402823466e38f ? __fmaf_rn(e, r, q) : q;
+}
+
+// One axis around a cell: the centres of the cell and its two neighbours, the
+// two intervals between them and their reciprocals (fluid.py:2407-2433 for a
+// point that stays in one of them).
+struct AxisNear {
+  int i, n;
+  float cm, c0, cp, dm, dp, rm, rp;
+};
+
+__device__ __forceinline__ AxisNear axis_near(const float* __restrict__ centers, int i, int n) {
+  AxisNear a;
+  a.i = i;
+  a.n = n;
+  a.c0 = __ldg(centers + i);
+  a.cm = i > 0 ? __ldg(centers + i - 1) : a.c0;
+  a.cp = i < n - 1 ? __ldg(centers + i + 1) : a.c0;
+  a.dm = fmaxf(__fsub_rn(a.c0, a.cm), 1.0e-18f);
+  a.dp = fmaxf(__fsub_rn(a.cp, a.c0), 1.0e-18f);
+  a.rm = __frcp_rn(a.dm);
+  a.rp = __frcp_rn(a.dp);
+  return a;
+}
+
+__device__ __forceinline__ float coord_near(const AxisNear& a, float v, const float* __restrict__ faces,
+                                            const float* __restrict__ centers) {
+  if (v >= a.c0 && v < a.cp) return __fadd_rn((float)a.i, div_by(__fsub_rn(v, a.c0), a.dp, a.rp));
+  if (v >= a.cm && v < a.c0) return __fadd_rn((float)(a.i - 1), div_by(__fsub_rn(v, a.cm), a.dm, a.rm));
+  return axis_coord(v, faces, centers, a.n, a.i);
+}
+
+constexpr int kPK = 32, kPJ = 8;  // cells per block along k and j
+constexpr int kPW = kPK + 2, kPH = kPJ + 2;
+
+// sample_prev from the block's tile, whose cell (0, 0, 0) is grid cell
+// (o0, o1, o2); a departure point that leaves the tile reads the grid.
+template <int kNI>
+__device__ __forceinline__ void sample_tile(const LevelDev& L, const float* __restrict__ vp, const float4* tile,
+                                            int o0, int o1, int o2, float gx, float gy, float gz, const float fb[3],
+                                            float out[3]) {
+  const int i0 = min(max((int)floorf(gx), 0), L.nx - 2);
+  const int j0 = min(max((int)floorf(gy), 0), L.ny - 2);
+  const int k0 = min(max((int)floorf(gz), 0), L.nz - 2);
+  const int li = i0 - o0, lj = j0 - o1, lk = k0 - o2;
+  if ((unsigned)li > (unsigned)kNI || (unsigned)lj > (unsigned)kPJ || (unsigned)lk > (unsigned)kPK) {
+    sample_prev(L, vp, gx, gy, gz, fb, out);
     return;
   }
-  const int64_t sx = (int64_t)L.ny * L.nz, sy = L.nz;
-  const float cen[3] = {__ldg(vp + 3 * c), __ldg(vp + 3 * c + 1), __ldg(vp + 3 * c + 2)};
-  const float x = __ldg(A.cx + i), y = __ldg(A.cy + j), z = __ldg(A.cz + k);
-  float tr[3] = {cen[0], cen[1], cen[2]};
-  if (rk2) {
-    float hd = __fmul_rn(0.5f, dt);
-    float mx = __fsub_rn(x, __fmul_rn(hd, cen[0]));
-    float my = __fsub_rn(y, __fmul_rn(hd, cen[1]));
-    float mz = __fsub_rn(z, __fmul_rn(hd, cen[2]));
-    sample_prev(L, vp, axis_coord(mx, A.fx, A.cx, L.nx, i), axis_coord(my, A.fy, A.cy, L.ny, j),
-                axis_coord(mz, A.fz, A.cz, L.nz, k), cen, tr);
+  const float tx = fminf(fmaxf(__fsub_rn(gx, (float)i0), 0.0f), 1.0f);
+  const float ty = fminf(fmaxf(__fsub_rn(gy, (float)j0), 0.0f), 1.0f);
+  const float tz = fminf(fmaxf(__fsub_rn(gz, (float)k0), 0.0f), 1.0f);
+  const float wx[2] = {__fsub_rn(1.0f, tx), tx}, wy[2] = {__fsub_rn(1.0f, ty), ty}, wz[2] = {__fsub_rn(1.0f, tz), tz};
+  const float4* at = tile + (li * kPH + lj) * kPW + lk;
+  float v0 = 0.f, v1 = 0.f, v2 = 0.f, fw = 0.f;
+#pragma unroll
+  for (int oi = 0; oi < 2; ++oi)
+#pragma unroll
+    for (int oj = 0; oj < 2; ++oj) {
+      const float wxy = __fmul_rn(wx[oi], wy[oj]);
+#pragma unroll
+      for (int ok = 0; ok < 2; ++ok) {
+        // cells off the fluid set are zero in the tile and weigh nothing
+        const float4 c = at[(oi * kPH + oj) * kPW + ok];
+        const float w = __fmul_rn(__fmul_rn(wxy, wz[ok]), c.w);
+        v0 = __fadd_rn(v0, __fmul_rn(w, c.x));
+        v1 = __fadd_rn(v1, __fmul_rn(w, c.y));
+        v2 = __fadd_rn(v2, __fmul_rn(w, c.z));
+        fw = __fadd_rn(fw, w);
+      }
+    }
+  if (fw > 1.0e-12f) {
+    const float r = __frcp_rn(fw);
+    out[0] = div_by(v0, fw, r);
+    out[1] = div_by(v1, fw, r);
+    out[2] = div_by(v2, fw, r);
+  } else {
+    out[0] = fb[0];
+    out[1] = fb[1];
+    out[2] = fb[2];
   }
-  float bx = __fsub_rn(x, __fmul_rn(dt, tr[0]));
-  float by = __fsub_rn(y, __fmul_rn(dt, tr[1]));
-  float bz = __fsub_rn(z, __fmul_rn(dt, tr[2]));
-  float adv[3];
-  sample_prev(L, vp, axis_coord(bx, A.fx, A.cx, L.nx, i), axis_coord(by, A.fy, A.cy, L.ny, j),
-              axis_coord(bz, A.fz, A.cz, L.nz, k), cen, adv);
-  const float dtnu = __fmul_rn(dt, nu);
-  const float icx = __ldg(L.cdx_f + i), icy = __ldg(L.cdy_f + j), icz = __ldg(L.cdz_f + k);
-  const float icxp = (i < L.nx - 1) ? __ldg(L.cdx_f + i + 1) : 1.0f;
+}
+
+// fluid.py:2447-2513 _predict_kernel.  A block of 32 x 8 threads takes kNI
+// planes of a 32 (k) x 8 (j) column tile and first stages the previous
+// velocity of the tile and its one-cell halo in shared memory, one float4 per
+// cell (u, v, w, 1 on fluid cells; zero elsewhere): the sixteen trilinear
+// corners of a departure point and the Laplacian's neighbours are then one
+// 16-byte shared load each instead of three strided global loads and a mask
+// byte, and a point moves less than a cell in all but violent steps.  The
+// divisors (widths, centre distances) are per axis, so their reciprocals are
+// formed once per thread or plane and the quotients by div_by.  Per-cell
+// global loads and full divisions took 955 us on a 256^3 grid with rk2 (25
+// bytes a cell: 64 us at the copy rate), this takes 669 us: the issue slots of
+// the correctly rounded f32 arithmetic bound both.
+template <int kNI>
+__global__ void __launch_bounds__(kPK* kPJ, 3) k_predict(LevelDev L, efsi_grid_axes A, const float* __restrict__ vp,
+                                                      float dt, float nu, int rk2, float* __restrict__ vel) {
+  extern __shared__ float4 ptile[];
+  const int o0 = (int)blockIdx.z * kNI - 1, o1 = (int)blockIdx.y * kPJ - 1, o2 = (int)blockIdx.x * kPK - 1;
+  for (int e = (int)(threadIdx.y * kPK + threadIdx.x); e < (kNI + 2) * kPH * kPW; e += kPK * kPJ) {
+    const int row = e / kPW, lk = e - row * kPW, li = row / kPH, lj = row - li * kPH;
+    const int64_t c = cix(min(max(o0 + li, 0), L.nx - 1), min(max(o1 + lj, 0), L.ny - 1),
+                          min(max(o2 + lk, 0), L.nz - 1), L.ny, L.nz);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (__ldg(L.mask + c) & M_FLUID)
+      v = make_float4(__ldg(vp + 3 * c), __ldg(vp + 3 * c + 1), __ldg(vp + 3 * c + 2), 1.0f);
+    ptile[e] = v;
+  }
+  __syncthreads();
+  const int j = o1 + 1 + (int)threadIdx.y, k = o2 + 1 + (int)threadIdx.x;
+  if (j >= L.ny || k >= L.nz) return;
+  const AxisNear ay = axis_near(A.cy, j, L.ny), az = axis_near(A.cz, k, L.nz);
+  const float dtnu = __fmul_rn(dt, nu), hd = __fmul_rn(0.5f, dt);
+  const float icy = __ldg(L.cdy_f + j), icz = __ldg(L.cdz_f + k);
   const float icyp = (j < L.ny - 1) ? __ldg(L.cdy_f + j + 1) : 1.0f;
   const float iczp = (k < L.nz - 1) ? __ldg(L.cdz_f + k + 1) : 1.0f;
-  const float wxi = __ldg(L.wx + i), wyj = __ldg(L.wy + j), wzk = __ldg(L.wz + k);
+  const float wyj = __ldg(L.wy + j), wzk = __ldg(L.wz + k);
+  const float ry = __frcp_rn(icy), rz = __frcp_rn(icz), ryp = __frcp_rn(icyp), rzp = __frcp_rn(iczp);
+  const float rwy = __frcp_rn(wyj), rwz = __frcp_rn(wzk);
+#pragma unroll 1
+  for (int q = 0; q < kNI; ++q) {
+    const int i = o0 + 1 + q;
+    if (i >= L.nx) return;
+    const int64_t c = cix(i, j, k, L.ny, L.nz);
+    const unsigned m = __ldg(L.mask + c);
+    if (m & M_SOLID) {
+      vel[3 * c] = vel[3 * c + 1] = vel[3 * c + 2] = 0.0f;
+      continue;
+    }
+    const float4* at = ptile + ((q + 1) * kPH + (int)threadIdx.y + 1) * kPW + (int)threadIdx.x + 1;
+    float4 own = *at;
+    if (!(m & M_FLUID)) own = make_float4(__ldg(vp + 3 * c), __ldg(vp + 3 * c + 1), __ldg(vp + 3 * c + 2), 0.0f);
+    const float cen[3] = {own.x, own.y, own.z};
+    const AxisNear ax = axis_near(A.cx, i, L.nx);
+    float tr[3] = {cen[0], cen[1], cen[2]};
+    if (rk2)
+      sample_tile<kNI>(L, vp, ptile, o0, o1, o2,
+                       coord_near(ax, __fsub_rn(ax.c0, __fmul_rn(hd, cen[0])), A.fx, A.cx),
+                       coord_near(ay, __fsub_rn(ay.c0, __fmul_rn(hd, cen[1])), A.fy, A.cy),
+                       coord_near(az, __fsub_rn(az.c0, __fmul_rn(hd, cen[2])), A.fz, A.cz), cen, tr);
+    float adv[3];
+    sample_tile<kNI>(L, vp, ptile, o0, o1, o2, coord_near(ax, __fsub_rn(ax.c0, __fmul_rn(dt, tr[0])), A.fx, A.cx),
+                     coord_near(ay, __fsub_rn(ay.c0, __fmul_rn(dt, tr[1])), A.fy, A.cy),
+                     coord_near(az, __fsub_rn(az.c0, __fmul_rn(dt, tr[2])), A.fz, A.cz), cen, adv);
+    const float icx = __ldg(L.cdx_f + i), icxp = (i < L.nx - 1) ? __ldg(L.cdx_f + i + 1) : 1.0f;
+    const float wxi = __ldg(L.wx + i);
+    const float rx = __frcp_rn(icx), rxp = __frcp_rn(icxp), rwx = __frcp_rn(wxi);
+    // a neighbour behind an open face is a fluid cell: its tile value is its velocity
+    const float4 xm = at[-kPH * kPW], xp = at[kPH * kPW], ym = at[-kPW], yp = at[kPW], zm = at[-1], zp = at[1];
+    const float nb[6][3] = {{xm.x, xm.y, xm.z}, {xp.x, xp.y, xp.z}, {ym.x, ym.y, ym.z},
+                            {yp.x, yp.y, yp.z}, {zm.x, zm.y, zm.z}, {zp.x, zp.y, zp.z}};
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    float fxb = 0.f, fxf = 0.f, fyb = 0.f, fyf = 0.f, fzb = 0.f, fzf = 0.f;
-    if (m & M_XM) fxb = __fdiv_rn(__fsub_rn(cen[a], __ldg(vp + 3 * (c - sx) + a)), icx);
-    if (m & M_XP) fxf = __fdiv_rn(__fsub_rn(__ldg(vp + 3 * (c + sx) + a), cen[a]), icxp);
-    if (m & M_YM) fyb = __fdiv_rn(__fsub_rn(cen[a], __ldg(vp + 3 * (c - sy) + a)), icy);
-    if (m & M_YP) fyf = __fdiv_rn(__fsub_rn(__ldg(vp + 3 * (c + sy) + a), cen[a]), icyp);
-    if (m & M_ZM) fzb = __fdiv_rn(__fsub_rn(cen[a], __ldg(vp + 3 * (c - 1) + a)), icz);
-    if (m & M_ZP) fzf = __fdiv_rn(__fsub_rn(__ldg(vp + 3 * (c + 1) + a), cen[a]), iczp);
-    float lap = __fadd_rn(__fadd_rn(__fdiv_rn(__fsub_rn(fxf, fxb), wxi), __fdiv_rn(__fsub_rn(fyf, fyb), wyj)),
-                          __fdiv_rn(__fsub_rn(fzf, fzb), wzk));
-    vel[3 * c + a] = __fadd_rn(adv[a], __fmul_rn(dtnu, lap));
+    for (int a = 0; a < 3; ++a) {
+      float fxb = 0.f, fxf = 0.f, fyb = 0.f, fyf = 0.f, fzb = 0.f, fzf = 0.f;
+      if (m & M_XM) fxb = div_by(__fsub_rn(cen[a], nb[0][a]), icx, rx);
+      if (m & M_XP) fxf = div_by(__fsub_rn(nb[1][a], cen[a]), icxp, rxp);
+      if (m & M_YM) fyb = div_by(__fsub_rn(cen[a], nb[2][a]), icy, ry);
+      if (m & M_YP) fyf = div_by(__fsub_rn(nb[3][a], cen[a]), icyp, ryp);
+      if (m & M_ZM) fzb = div_by(__fsub_rn(cen[a], nb[4][a]), icz, rz);
+      if (m & M_ZP) fzf = div_by(__fsub_rn(nb[5][a], cen[a]), iczp, rzp);
+      const float lap = __fadd_rn(__fadd_rn(div_by(__fsub_rn(fxf, fxb), wxi, rwx), div_by(__fsub_rn(fyf, fyb), wyj, rwy)),
+                                  div_by(__fsub_rn(fzf, fzb), wzk, rwz));
+      vel[3 * c + a] = __fadd_rn(adv[a], __fmul_rn(dtnu, lap));
+    }
   }
+}
+
+template <int kNI>
+static void launch_predict(const LevelDev& L, const efsi_grid_axes& axes, const float* vp, float dt, float nu,
+                           int rk2, float* vel, cudaStream_t s) {
+  const dim3 grid((unsigned)((L.nz + kPK - 1) / kPK), (unsigned)((L.ny + kPJ - 1) / kPJ),
+                  (unsigned)((L.nx + kNI - 1) / kNI));
+  constexpr size_t smem = sizeof(float4) * (kNI + 2) * kPH * kPW;
+  if (smem > 48 * 1024)
+    cudaFuncSetAttribute(k_predict<kNI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  EFSI_COUNTED k_predict<kNI><<<grid, dim3(kPK, kPJ), smem, s>>>(L, axes, vp, dt, nu, rk2, vel);
 }
 
 // fluid.py:3494-3565 divergence statistics: max |v|, sum v^2, count.
@@ -592,9 +732,17 @@ int efsi_predict(efsi_fv_plan* P, const efsi_grid_axes* axes, const float* veloc
   EFSI_ARG_CHECK(axes != nullptr && velocity_prev != nullptr && velocity != nullptr && velocity != velocity_prev,
                  "predict needs distinct velocity and velocity_prev buffers");
   LevelDev L = level_dev(P, 0);
-  const Shape3& S = P->lv[0].shape;
-  EFSI_TIMED(KF_PREDICT, 25.0 * P->lv[0].n, as_stream(stream),
-             EFSI_COUNTED k_predict<<<S.grid, S.block, 0, as_stream(stream)>>>(L, *axes, velocity_prev, dt, nu, rk2, velocity));
+  cudaStream_t s = as_stream(stream);
+  // six planes a block (42 KB, three blocks per SM) read each tile 1.8 times
+  // over; two planes read it 2.7 times over but give a small grid three times
+  // the blocks, which is what counts until the SMs are full
+  const int64_t blocks6 = (int64_t)((L.nz + kPK - 1) / kPK) * ((L.ny + kPJ - 1) / kPJ) * ((L.nx + 5) / 6);
+  if (blocks6 >= 4 * 148)
+    EFSI_TIMED(KF_PREDICT, 25.0 * P->lv[0].n, s,
+               launch_predict<6>(L, *axes, velocity_prev, dt, nu, rk2, velocity, s));
+  else
+    EFSI_TIMED(KF_PREDICT, 25.0 * P->lv[0].n, s,
+               launch_predict<2>(L, *axes, velocity_prev, dt, nu, rk2, velocity, s));
   EFSI_LAUNCH_CHECK();
   return EFSI_OK;
 }

@@ -9,6 +9,23 @@ from oracle import oracle as orc
 pytestmark = pytest.mark.gpu
 
 
+def _rel(a, b):
+    a = np.asarray(a, np.float64).ravel()
+    b = np.asarray(b, np.float64).ravel()
+    return float(np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-300))
+
+
+def _grid(nodes, graded):
+    from easyfsi_b200.grid import CartesianGrid
+    from easyfsi_b200.scenarios import graded_axis_widths
+
+    if not graded:
+        return CartesianGrid.uniform(bounds_min_m=(0.0, 0.0, 0.0), bounds_max_m=(1.0, 1.0, 1.0), grid_nodes=nodes)
+    return CartesianGrid(bounds_min_m=(0.0, 0.0, 0.0), cell_widths_x_m=graded_axis_widths(nodes[0], 0.0, 1.0, 0.3, 0.7),
+                         cell_widths_y_m=graded_axis_widths(nodes[1], 0.0, 1.0, 0.3, 0.7),
+                         cell_widths_z_m=graded_axis_widths(nodes[2], 0.0, 1.0, 0.2, 0.8))
+
+
 # ---------------------------------------------------------------------------
 # far nodes of the immersed-boundary search
 # ---------------------------------------------------------------------------
@@ -80,3 +97,37 @@ def test_far_nodes_match_the_all_pairs_oracle(bands, slivers, triangles, nodes):
                      (search.node_interior_fluid_point_m, "interior_point"),
                      (search.node_projection_marker_weights, "projection_weights")):
         np.testing.assert_allclose(got.to_numpy(), ref[key], rtol=0.0, atol=1e-6, err_msg=key)
+
+
+# ---------------------------------------------------------------------------
+# predictor tiles
+# ---------------------------------------------------------------------------
+
+
+@pytest.mark.parametrize("nodes,graded,dt", [
+    ((4, 4, 4), False, 1.0e-2),
+    ((9, 17, 33), True, 1.0e-2),    # one past a tile along j and k
+    ((13, 8, 70), True, 2.0e-1),    # departure points several cells away
+    ((50, 65, 96), False, 1.0e-3),  # six planes a block
+])
+@pytest.mark.parametrize("rk2", [False, True])
+def test_predictor_matches_the_oracle(nodes, graded, dt, rk2):
+    """Random velocities and masked cells; the tile's arithmetic rounds as the
+    oracle's (quotients by a corrected reciprocal), so the bound is half a
+    unit in the last place of the result, 2^-24."""
+    from easyfsi_b200.fluid import CartesianFluidSolver, FluidDomainSpec
+
+    grid = _grid(nodes, graded)
+    fl = CartesianFluidSolver(FluidDomainSpec((0, 0, 0), grid.bounds_max_m, None, 1000.0, 1.0e-2, 1.0e-3,
+                                              cartesian_grid=grid))
+    ofl = orc.OracleFluid(grid, rho=1000.0, mu=1.0e-2)
+    rng = np.random.default_rng(nodes[2])
+    obs = (rng.random(nodes) < 0.05).astype(np.int32)
+    vel = (0.3 * rng.normal(size=nodes + (3,))).astype(np.float32)
+    fl.obstacle.from_numpy(obs)
+    fl.velocity.from_numpy(vel)
+    ofl.obstacle[...] = obs
+    ofl.velocity[...] = vel
+    fl.predict(dt, advection_scheme="rk2" if rk2 else "euler")
+    ofl.predict(dt, rk2=rk2)
+    assert _rel(fl.velocity.to_numpy(), ofl.velocity) <= 2.0**-24

@@ -2,20 +2,37 @@
 // (tcgen05), for the learned preconditioner's U-Net.
 //
 // Forward (and, with flipped / transposed weights, the input gradient) is an
-// implicit GEMM: D[v][co] = sum_t sum_ci X[v + off(t)][ci] W[co][t][ci], with
-// M = 128 consecutive voxels per CTA, N = Cout (16..256, a multiple of 16) and
-// K = 27 taps x Cin (Cin a multiple of 16).  Per tap the 128 x Cin slice of
-// the im2col matrix (zero outside the volume) and the Cout x Cin slice of the
-// weights are copied by the CTA's threads (cp.async, 16 bytes each, zero
-// filled outside the volume) into shared memory in the canonical no-swizzle
-// K-major layout (8-row x 16-byte core matrices: SBO = 128 bytes between
-// 8-row groups, LBO = rows x 16 bytes between 8-element K chunks), through a
-// ring of kStages stages, so the copies of the next kAhead taps are in flight
-// while one elected thread issues tcgen05.mma.kind::f16 (BF16
-// operands, FP32 accumulator in tensor memory) per 16-channel K step of the
-// current tap and commits to the stage's mbarrier.  The epilogue reads the accumulator with tcgen05.ld (warp w owns
-// lanes 32w..32w+31 = voxels), adds the bias, applies ReLU if asked and
-// stores BF16 (and optionally FP32).
+// implicit GEMM: D[v][co] = sum_t sum_ci X[v + off(t)][ci] W[co][t][ci].
+// A CTA owns a box of bj lines x bz voxels along z of bi planes along x and nt
+// of the output channels.  It keeps its channels' weights of all 27 taps and a
+// ring of input planes, each with a one-voxel halo in j and k, in shared
+// memory in the canonical no-swizzle K-major layout (8 rows x 16 bytes per
+// core matrix): the voxels of a haloed plane, line after line, are the rows,
+// 16 bytes apart, one run of rows per 8-channel chunk.  A tap is then the
+// same rows shifted by di planes, dj lines and dk rows, which is only another
+// start address in the MMA's descriptor: every voxel is copied to shared
+// memory once per plane ring and not once per tap, and the 27 taps of a plane
+// are issued back to back.  M = 128 consecutive rows (the halo rows among
+// them compute values that are not stored), N = nt, K = 16 channels per MMA.
+// One elected thread issues tcgen05.mma.kind::f16 (BF16 operands, FP32
+// accumulator in tensor memory) and commits a plane's MMAs to an mbarrier;
+// meanwhile all threads copy the plane after next (cp.async, zero filled
+// outside the volume) and write the previous plane's result: tcgen05.ld (warp
+// w owns lanes 32w..32w+31 = rows), bias, ReLU, BF16 (and optionally FP32).
+//
+// What bounds it: an MMA of N = 16..64 reads its 4 KB A operand from shared
+// memory in about 32 cycles, more than its tensor-core time, so the tensor
+// pipe cannot fill at these channel counts; the box is chosen (conv_tile) so
+// that enough CTAs run and few halo rows are computed.  With the voxels copied
+// again for every tap, a network forward at 64 x 72 x 128 took 1.89 ms; it takes
+// 1.14 ms now.
+//
+// The weight gradient dW[co][t][ci] = sum_v dY[v][co] X[v + off(t)][ci] reads
+// the same images as MN-major operands (rows = voxels = K): A is the three
+// planes' chunks of X side by side, so M runs over (di, ci), N over co, and a
+// tap's (dj, dk) is again a row shift.
+// On the FP32 pipes it was 14.0 of the 18.2 ms of the gradients of four 32^3
+// crops; all of those take 5.1 ms now.
 //
 // Every mbarrier wait is bounded; a wait that gives up sets the caller's
 // error word, waits (bounded) for the MMAs in flight and frees the tensor
@@ -25,16 +42,14 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 namespace efsi {
 namespace conv {
 
-constexpr int kTileM = 128;          // voxels per CTA (MMA M)
+constexpr int kTileM = 128;          // rows per MMA
 constexpr int kThreads = 128;        // 4 warps: one TMEM lane quadrant each
-constexpr int kStages = 4;           // taps in the shared-memory ring
-constexpr int kLag = 2;              // a stage is refilled once the MMAs of kLag taps ago are done
-constexpr int kAhead = kStages - kLag;  // taps whose copies are in flight ahead of the current one
 constexpr long long kWaitLimit = 4000000000LL;  // ~2 s of clock64
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -49,9 +64,11 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint
   return d;
 }
 
-// Instruction descriptor of kind::f16: BF16 A and B (both K-major), FP32 D.
-__host__ __device__ constexpr uint32_t idesc_bf16(int m, int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+// Instruction descriptor of kind::f16: BF16 A and B (both K-major, or both
+// MN-major), FP32 D.
+__host__ __device__ constexpr uint32_t idesc_bf16(int m, int n, bool mn_major = false) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (mn_major ? (3u << 15) : 0u) | ((uint32_t)(n >> 3) << 17) |
+         ((uint32_t)(m >> 4) << 24);
 }
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar) {
@@ -119,10 +136,20 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
   for (int q = 0; q < 16; ++q) v[q] = __uint_as_float(r[q]);
 }
 
+// A volume's channels-last input, [n][cin]; with `coarse` the first ca channels
+// come from the parent voxels of a ceil-halved volume (nearest-neighbour
+// upsampling) and the other cin - ca from x, without the concatenation being
+// stored.
+struct ConvInput {
+  const __nv_bfloat16* x;
+  const __nv_bfloat16* coarse;
+  int ca;
+};
+
 struct ConvArgs {
   int nx, ny, nz;
-  int cin, cout;                 // multiples of 16; cout <= 256
-  const __nv_bfloat16* x;        // [n][cin]
+  int cin, cout;                 // multiples of 16
+  ConvInput in;
   const __nv_bfloat16* w;        // [cout][27][cin]
   const float* bias;             // [cout] or null
   int relu;                      // apply ReLU in the epilogue
@@ -131,149 +158,433 @@ struct ConvArgs {
   int* error;                    // set to 1 when a wait gives up
 };
 
-// Bytes of dynamic shared memory for one launch (kStages stages of A and B).
-__host__ __device__ inline int conv_smem_bytes(int cin, int cout) {
-  const int a = kTileM * cin * 2, b = cout * cin * 2;
-  return kStages * (a + b) + 128;
-}
+// The box of one CTA and its shared-memory layout.
+struct ConvTile {
+  int bz, zp;        // output voxels per line, rows per line (bz + 2)
+  int bj, bi;        // lines per plane, planes
+  int nt;            // output channels
+  int mt;            // 128-row MMA tiles per plane
+  int slots;         // planes in the ring: 3 (bi == 1) or 4
+  int nzb, njb, nib; // boxes along z, y, x
+  int cs;            // bytes between the chunks of the input
+  int woff;          // byte offset of the weights
+  int smem;          // dynamic shared memory
+  unsigned cols;     // tensor-memory columns
+};
 
-__host__ __device__ inline uint32_t tmem_columns(int cout) {
+constexpr int kGuard = 128;  // bytes before the first row (tap -1 of row 0)
+
+__host__ __device__ inline uint32_t tmem_columns(int n) {
   uint32_t c = 32;
-  while ((int)c < cout) c <<= 1;
+  while ((int)c < n) c <<= 1;
   return c;
 }
 
-__global__ void __launch_bounds__(kThreads) k_conv3d_tc(ConvArgs A) {
+// 16-byte chunk c of voxel (i, j, k), or zeros outside the volume.
+__device__ __forceinline__ void copy_chunk(unsigned char* dst, const ConvInput& in, int nx, int ny, int nz, int cin,
+                                           int i, int j, int k, int c) {
+  const bool ok = i >= 0 && i < nx && j >= 0 && j < ny && k >= 0 && k < nz;
+  const __nv_bfloat16* src = in.x;
+  if (ok) {
+    if (c * 8 < in.ca)
+      src = in.coarse +
+            (((int64_t)(i >> 1) * ((ny + 1) >> 1) + (j >> 1)) * ((nz + 1) >> 1) + (k >> 1)) * in.ca + c * 8;
+    else
+      src = in.x + (((int64_t)i * ny + j) * nz + k) * (cin - in.ca) + (c * 8 - in.ca);
+  }
+  cp_async16(dst, src, ok ? 16 : 0);
+}
+
+__device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(cols)
+               : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_free(uint32_t tmem, uint32_t cols) {
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+}
+
+__global__ void __launch_bounds__(kThreads) k_conv3d_tc(ConvArgs A, ConvTile T) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t bars[kStages];
+  __shared__ __align__(8) uint64_t bars[2];
   __shared__ uint32_t tmem_slot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int cin = A.cin, cout = A.cout;
-  const int a_bytes = kTileM * cin * 2, b_bytes = cout * cin * 2;
-  const int stage_bytes = a_bytes + b_bytes;
-  const uint32_t lbo_a = (kTileM / 8) * 128, lbo_b = (uint32_t)(cout / 8) * 128;
-  const uint32_t ncols = tmem_columns(cout);
-  const int64_t n = (int64_t)A.nx * A.ny * A.nz;
-  const int64_t v0 = (int64_t)blockIdx.x * kTileM;
+  const int cin = A.cin, kch = cin / 8, nt = T.nt, zp = T.zp;
+  int b = blockIdx.x;
+  const int z0 = (b % T.nzb) * T.bz;
+  b /= T.nzb;
+  const int j0 = (b % T.njb) * T.bj, ib = (b / T.njb) * T.bi, ie = min(A.nx, ib + T.bi);
+  const int n0 = blockIdx.y * nt;
+  const int rows = (T.bj + 2) * zp, plane_bytes = rows * 16;
+  unsigned char* sx = smem_raw + kGuard;
+  unsigned char* sw = smem_raw + T.woff;
 
   if (tid == 0) {
-    for (int q = 0; q < kStages; ++q) mbar_init(&bars[q]);
+    mbar_init(&bars[0]);
+    mbar_init(&bars[1]);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                 "r"(ncols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  if (warp == 0) tmem_alloc(&tmem_slot, T.cols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
 
-  // this thread's voxel row of the im2col slice
-  const int64_t v = v0 + tid;
-  int vi = 0, vj = 0, vk = 0;
-  if (v < n) {
-    vk = (int)(v % A.nz);
-    const int64_t ij = v / A.nz;
-    vj = (int)(ij % A.ny);
-    vi = (int)(ij / A.ny);
-  }
-  const int kchunks = cin / 8;
-  // copies of tap t into its stage: the thread's A row and a share of B
-  auto issue = [&](int t) {
-    unsigned char* sa = smem_raw + (t % kStages) * stage_bytes;
-    unsigned char* sb = sa + a_bytes;
-    const int di = t / 9 - 1, dj = (t / 3) % 3 - 1, dk = t % 3 - 1;
-    const int ii = vi + di, jj = vj + dj, kk = vk + dk;
-    const bool in = v < n && ii >= 0 && ii < A.nx && jj >= 0 && jj < A.ny && kk >= 0 && kk < A.nz;
-    const __nv_bfloat16* src = in ? A.x + (((int64_t)ii * A.ny + jj) * A.nz + kk) * cin : A.x;
-    unsigned char* dst = sa + (tid >> 3) * 128 + (tid & 7) * 16;
-    for (int c = 0; c < kchunks; ++c) cp_async16(dst + c * lbo_a, src + (in ? c * 8 : 0), in ? 16 : 0);
-    for (int q = tid; q < cout * kchunks; q += kThreads) {
-      const int co = q / kchunks, c = q - co * kchunks;
-      cp_async16(sb + c * lbo_b + (co >> 3) * 128 + (co & 7) * 16, A.w + ((int64_t)co * 27 + t) * cin + c * 8, 16);
+  // plane p lives in slot (p - ib + 1) % slots
+  auto load_plane = [&](int p) {
+    unsigned char* dst = sx + ((p - ib + 1) % T.slots) * plane_bytes;
+    for (int e = tid; e < rows * kch; e += kThreads) {
+      const int row = e / kch, c = e - row * kch;
+      const int line = row / zp, z = row - line * zp;
+      copy_chunk(dst + c * T.cs + row * 16, A.in, A.nx, A.ny, A.nz, cin, p, j0 - 1 + line, z0 - 1 + z, c);
     }
   };
-  const uint32_t idesc = idesc_bf16(kTileM, cout);
-  // prologue: taps 0 .. kAhead - 1 in flight (one commit group per tap)
-  for (int t = 0; t < kAhead; ++t) {
-    issue(t);
-    cp_async_commit();
+  for (int q = tid; q < 27 * nt * kch; q += kThreads) {
+    const int c = q % kch, r = q / kch, t = r % 27, co = r / 27;
+    cp_async16(sw + ((t * kch + c) * nt + co) * 16, A.w + ((int64_t)(n0 + co) * 27 + t) * cin + c * 8, 16);
   }
-  bool ok = true, good = true;
-  for (int t = 0; t < 27; ++t) {
-    // this thread's copies of tap t have landed once at most kAhead - 1
-    // newer groups are pending; the block decides together whether to go on
-    cp_async_wait<kAhead - 1>();
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    if (!__syncthreads_and(good)) {
-      ok = false;
-      break;
-    }
-    if (tid == 0) {
-      tc_fence_after();
-      const uint32_t a0 = smem_u32(smem_raw + (t % kStages) * stage_bytes);
-      const uint32_t b0 = a0 + a_bytes;
-      for (int ks = 0; ks < cin / 16; ++ks) {
-        const uint64_t ad = umma_desc(a0 + ks * 2 * lbo_a, lbo_a, 128);
-        const uint64_t bd = umma_desc(b0 + ks * 2 * lbo_b, lbo_b, 128);
-        tc_mma(tmem, ad, bd, idesc, (t > 0 || ks > 0) ? 1 : 0);
-      }
-      tc_commit(&bars[t % kStages]);
-    }
-    // refill the stage of tap t - kLag with tap t + kAhead once the MMAs of
-    // tap t - kLag have read it (issued kLag iterations ago, so the wait is
-    // normally already over)
-    const int tn = t + kAhead;
-    if (tn < 27) {
-      if (t >= kLag) good = mbar_wait_bounded(&bars[(t - kLag) % kStages], (unsigned)(((t - kLag) / kStages) & 1));
-      if (good) issue(tn);
-    }
-    cp_async_commit();  // one group per iteration, possibly empty
-  }
+  for (int p = ib - 1; p <= ib + 1; ++p) load_plane(p);
+  cp_async_commit();
   cp_async_wait<0>();
-  // the last commit covers every MMA issued before it
-  ok = __syncthreads_and(ok && mbar_wait_bounded(&bars[26 % kStages], (unsigned)((26 / kStages) & 1)));
-  tc_fence_after();
-  if (ok) {
-    const int64_t vr = v0 + warp * 32 + lane;
-    for (int c0 = 0; c0 < cout; c0 += 16) {
-      float acc[16];
-      tc_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, acc);
-      if (vr < n) {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncthreads();
+
+  const uint32_t idesc = idesc_bf16(kTileM, nt);
+  // the 27 taps of output plane i into accumulator set `buf`
+  auto issue = [&](int i, int buf) {
+    tc_fence_after();
+    for (int m = 0; m < T.mt; ++m) {
+      const uint32_t acc = tmem + (uint32_t)((buf * T.mt + m) * nt);
+      for (int t = 0; t < 27; ++t) {
+        const int di = t / 9 - 1, dj = (t / 3) % 3 - 1, dk = t % 3 - 1;
+        const uint32_t a0 = smem_u32(sx) + (uint32_t)(((i + di - ib + 1) % T.slots) * plane_bytes) +
+                            (uint32_t)((m * kTileM + (1 + dj) * zp + dk) * 16);
+        const uint32_t b0 = smem_u32(sw) + (uint32_t)(t * kch * nt * 16);
+        for (int ks = 0; ks < kch / 2; ++ks)
+          tc_mma(acc, umma_desc(a0 + (uint32_t)(2 * ks * T.cs), (uint32_t)T.cs, 128),
+                 umma_desc(b0 + (uint32_t)(2 * ks * nt * 16), (uint32_t)(nt * 16), 128), idesc,
+                 (t > 0 || ks > 0) ? 1 : 0);
+      }
+    }
+    tc_commit(&bars[buf]);
+  };
+  auto epilogue = [&](int i, int buf) {
+    tc_fence_after();
+    for (int m = 0; m < T.mt; ++m) {
+      const int row = m * kTileM + warp * 32 + lane;
+      const int line = row / zp, z = row - line * zp;
+      const int j = j0 + line, k = z0 + z - 1;
+      const bool in = line < T.bj && z >= 1 && z <= T.bz && j < A.ny && k < A.nz;
+      const int64_t at = (((int64_t)i * A.ny + j) * A.nz + k) * A.cout + n0;
+      for (int c0 = 0; c0 < nt; c0 += 16) {
+        float acc[16];
+        tc_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((buf * T.mt + m) * nt + c0), acc);
+        if (!in) continue;
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
-          float a = acc[q] + (A.bias != nullptr ? __ldg(A.bias + c0 + q) : 0.0f);
+          const float a = acc[q] + (A.bias != nullptr ? __ldg(A.bias + n0 + c0 + q) : 0.0f);
           acc[q] = A.relu ? fmaxf(a, 0.0f) : a;
         }
         if (A.y != nullptr) {
           __align__(16) __nv_bfloat16 hb[16];
 #pragma unroll
           for (int q = 0; q < 16; ++q) hb[q] = __float2bfloat16_rn(acc[q]);
-          uint4* dst = reinterpret_cast<uint4*>(A.y + vr * cout + c0);
+          uint4* dst = reinterpret_cast<uint4*>(A.y + at + c0);
           dst[0] = reinterpret_cast<const uint4*>(hb)[0];
           dst[1] = reinterpret_cast<const uint4*>(hb)[1];
         }
         if (A.yf != nullptr) {
-          float4* dst = reinterpret_cast<float4*>(A.yf + vr * cout + c0);
+          float4* dst = reinterpret_cast<float4*>(A.yf + at + c0);
 #pragma unroll
           for (int q = 0; q < 4; ++q) dst[q] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
         }
       }
     }
-  } else {
-    if (tid == 0) atomicExch(A.error, 1);
-    // drain: give the MMAs in flight a bounded chance to finish
-    for (int q = 0; q < kStages; ++q) mbar_wait_bounded(&bars[q], 0);
+    tc_fence_before();
+  };
+  // Plane i's MMAs run while plane i + 2 is copied and plane i - 1's result is
+  // written.  Plane i + 2 takes the slot of plane i - 2, which the MMAs of
+  // plane i - 1 read last; the rows past a plane's last line that an MMA tile
+  // also covers may see it arrive, and are not stored.
+  bool ok = true;
+  int last = -1;  // last plane whose MMAs were issued, from ib
+  for (int q = 0; q < ie - ib; ++q) {
+    if (tid == 0) issue(ib + q, q & 1);
+    last = q;
+    bool good = true;
+    if (q > 0) good = mbar_wait_bounded(&bars[(q - 1) & 1], (unsigned)(((q - 1) >> 1) & 1));
+    if (good && q + 1 < ie - ib) load_plane(ib + q + 2);
+    cp_async_commit();
+    // (the same for all lanes of a warp: tcgen05.ld is a warp's instruction;
+    // the exit is taken by all threads together, after the copies have landed)
+    good = __all_sync(0xffffffffu, good);
+    if (good && q > 0) epilogue(ib + q - 1, (q - 1) & 1);
+    cp_async_wait<0>();
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (!__syncthreads_and(good)) {
+      ok = false;
+      break;
+    }
+  }
+  const bool done = mbar_wait_bounded(&bars[last & 1], (unsigned)((last >> 1) & 1));
+  ok = __syncthreads_and(ok && done);
+  if (ok)
+    epilogue(ib + last, last & 1);
+  else if (tid == 0)
+    atomicExch(A.error, 1);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_free(tmem, T.cols);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Weight gradient: dw[co][t][ci] += sum_v dy[v][co] X[v + off(t)][ci].
+// ---------------------------------------------------------------------------
+struct WgradArgs {
+  int nx, ny, nz;
+  int cin, cout;            // multiples of 16
+  ConvInput in;
+  const __nv_bfloat16* dy;  // [n][cout]
+  float* dw;                // [cout][27][cin]
+  int* error;               // as in ConvArgs; null: dw[0] becomes NaN instead
+};
+
+// One CTA: one dj, `ndk` of the dk (grid y), mb of the 128-row blocks of
+// (di, ci) and nt output channels (grid z), boxes of bj lines x bz voxels of a
+// plane (grid x, strided).
+struct WgradTile {
+  int bz, zp, bj;
+  int rows;         // K rows of a box, bj * zp rounded up to 16
+  int nzb, njb;
+  int items;        // boxes
+  int ndk, mb, nmb, nt;
+  int cs, ds;       // bytes between the chunks of x and of dy
+  int doff;         // byte offset of dy
+  int smem;
+  unsigned cols;
+};
+
+__global__ void __launch_bounds__(kThreads) k_wgrad_tc(WgradArgs A, WgradTile T) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ uint32_t tmem_slot;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int cin = A.cin, kch = cin / 8, nch = T.nt / 8, zp = T.zp;
+  const int dj = (int)blockIdx.y % 3 - 1, dk0 = ((int)blockIdx.y / 3) * T.ndk - 1;
+  const int m0 = ((int)blockIdx.z % T.nmb) * T.mb, n0 = ((int)blockIdx.z / T.nmb) * T.nt;
+  // the chunks of the three planes this CTA's M blocks cover
+  const int g0 = m0 * (kTileM / 8), g1 = min(3 * kch, g0 + T.mb * (kTileM / 8));
+  unsigned char* sx = smem_raw + kGuard;
+  unsigned char* sd = smem_raw + T.doff;
+
+  if (tid == 0) {
+    mbar_init(&bar);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) tmem_alloc(&tmem_slot, T.cols);
+  // the row before the first and the row after the last of every chunk of x
+  // meet zero rows of dy: they only have to be finite
+  for (int g = tid; g < g1 - g0; g += kThreads) {
+    *reinterpret_cast<uint4*>(sx + g * T.cs - 16) = make_uint4(0u, 0u, 0u, 0u);
+    *reinterpret_cast<uint4*>(sx + g * T.cs + T.rows * 16) = make_uint4(0u, 0u, 0u, 0u);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot;
+  const uint32_t idesc = idesc_bf16(kTileM, T.nt, true);
+
+  bool ok = true;
+  int uses = 0;
+  for (int item = blockIdx.x; item < T.items; item += gridDim.x, ++uses) {
+    const int z0 = (item % T.nzb) * T.bz, rest = item / T.nzb;
+    const int j0 = (rest % T.njb) * T.bj, i = rest / T.njb;
+    // Row r of a box is voxel (line r / zp, z0 - 1 + r % zp): dy is zero on
+    // the halo columns and beyond the box, x of line j + dj is what it is
+    // there (zero outside the volume).
+    for (int e = tid; e < T.rows * (g1 - g0); e += kThreads) {
+      const int row = e / (g1 - g0), g = g0 + e - row * (g1 - g0);
+      const int line = row / zp, z = row - line * zp, di = g / kch - 1, c = g % kch;
+      copy_chunk(sx + (g - g0) * T.cs + row * 16, A.in, A.nx, A.ny, A.nz, cin, i + di,
+                 line < T.bj ? j0 + line + dj : -1, z0 - 1 + z, c);
+    }
+    for (int e = tid; e < T.rows * nch; e += kThreads) {
+      const int row = e / nch, c = e - row * nch;
+      const int line = row / zp, z = row - line * zp, j = j0 + line, k = z0 - 1 + z;
+      const bool in = line < T.bj && z >= 1 && z <= T.bz && j < A.ny && k < A.nz;
+      cp_async16(sd + c * T.ds + row * 16,
+                 in ? A.dy + (((int64_t)i * A.ny + j) * A.nz + k) * A.cout + n0 + c * 8 : A.dy, in ? 16 : 0);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (tid == 0) {
+      tc_fence_after();
+      for (int d = 0; d < T.ndk; ++d)
+        for (int m = 0; m < T.mb; ++m) {
+          const uint32_t acc = tmem + (uint32_t)((d * T.mb + m) * T.nt);
+          const uint32_t a0 = smem_u32(sx) + (uint32_t)(m * (kTileM / 8) * T.cs + (dk0 + d) * 16);
+          for (int r = 0; r < T.rows; r += 16)
+            tc_mma(acc, umma_desc(a0 + (uint32_t)(r * 16), 128, (uint32_t)T.cs),
+                   umma_desc(smem_u32(sd) + (uint32_t)(r * 16), 128, (uint32_t)T.ds), idesc,
+                   (uses > 0 || r > 0) ? 1 : 0);
+        }
+      tc_commit(&bar);
+    }
+    // the buffers are refilled for the next box once the MMAs have read them
+    const bool good = mbar_wait_bounded(&bar, (unsigned)(uses & 1));
+    if (!__syncthreads_and(good)) {
+      ok = false;
+      break;
+    }
+  }
+  if (!ok && tid == 0) {
+    if (A.error != nullptr)
+      atomicExch(A.error, 1);
+    else
+      A.dw[0] = __int_as_float(0x7fc00000);
+  }
+  if (ok && uses > 0) {
+    tc_fence_after();
+    for (int d = 0; d < T.ndk; ++d)
+      for (int m = 0; m < T.mb; ++m) {
+        const int row = (m0 + m) * kTileM + warp * 32 + lane;  // of (di, ci)
+        const int di = row / cin, ci = row - di * cin;
+        const int t = di * 9 + (dj + 1) * 3 + dk0 + d + 1;
+        for (int c0 = 0; c0 < T.nt; c0 += 16) {
+          float acc[16];
+          tc_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((d * T.mb + m) * T.nt + c0), acc);
+          if (di >= 3) continue;
+#pragma unroll
+          for (int q = 0; q < 16; ++q)
+            if (acc[q] != 0.0f) atomicAdd(A.dw + ((int64_t)(n0 + c0 + q) * 27 + t) * cin + ci, acc[q]);
+        }
+      }
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
+    tmem_free(tmem, T.cols);
   }
+}
+
+// ---------------------------------------------------------------------------
+// Tiles
+// ---------------------------------------------------------------------------
+constexpr int kMaxSmem = 222 * 1024;
+
+// Bytes between chunks: `bytes` rounded up to 64 past a multiple of 128, so
+// that the two chunks of neighbouring voxels' copies fall on different banks.
+inline int chunk_stride(int bytes) { return ((bytes + 127) & ~127) + 64; }
+
+// The CTAs of one SM together may not ask for more than its 512 tensor-memory
+// columns: the shared memory of a launch is raised until one more CTA than
+// they hold would not fit the SM.
+inline int smem_for(int bytes, unsigned cols) {
+  const int n = 512 / (int)cols;
+  return std::max(bytes, 228 * 1024 / (n + 1) + 1024);
+}
+
+// The box of a convolution: among the line lengths, MMA tiles per plane,
+// planes per CTA and channel splits that fit, the one with the least estimated
+// cycles -- per SM, the CTAs it gets in turn, each a fixed start (about 4000
+// cycles: launch, first copies, first MMA), its copies at 48 bytes a cycle and
+// its MMAs at 36 cycles (the A operand's shared-memory read).
+inline bool conv_tile(int nx, int ny, int nz, int cin, int cout, ConvTile& best) {
+  double least = 1e300;
+  const int kch = cin / 8;
+  for (int zcap : {62, 30, 14, 6})
+    for (int mt : {4, 2, 1})
+      for (int nt = std::min(cout, 128) / 16 * 16; nt >= 16; nt -= 16) {
+        if (cout % nt != 0) continue;
+        for (int bi : {16, 8, 4, 2, 1, 0}) {  // 0: one plane of one line, the least shared memory
+          if (bi > 1 && bi > nx) continue;
+          ConvTile t;
+          t.nt = nt;
+          t.mt = mt;
+          t.bi = std::max(bi, 1);
+          t.slots = bi > 1 ? 4 : 3;
+          t.nzb = (nz + zcap - 1) / zcap;
+          t.bz = (nz + t.nzb - 1) / t.nzb;
+          t.zp = t.bz + 2;
+          t.bj = bi == 0 ? 1 : std::min(ny, mt * kTileM / t.zp);
+          t.njb = (ny + t.bj - 1) / t.bj;
+          t.bj = (ny + t.njb - 1) / t.njb;
+          if ((mt - 1) * kTileM >= t.bj * t.zp) continue;  // a whole MMA tile without a row
+          t.nib = (nx + t.bi - 1) / t.bi;
+          const int rows = (t.bj + 2) * t.zp, w = 27 * kch * nt * 16;
+          t.cs = chunk_stride(t.slots * rows * 16);
+          // an MMA tile may reach past the last plane's rows: into the weights
+          t.woff = (kGuard + kch * t.cs + 127) & ~127;
+          const int used = t.woff + std::max(w, kTileM * 16 + 64);
+          t.cols = tmem_columns((bi > 1 ? 2 : 1) * mt * nt);
+          if (used > kMaxSmem || t.cols > 512) continue;
+          t.smem = smem_for(used, t.cols);
+          const int per_sm = std::max(1, 228 * 1024 / (t.smem + 1024));
+          const double ctas = (double)t.nzb * t.njb * t.nib * (cout / nt);
+          const double mma = (double)t.bi * mt * 27 * (kch / 2) * 36;
+          const double copy = (w + (t.bi + 2.0) * rows * cin * 2) / 48;
+          const double waves = std::max(1.0, std::ceil(ctas / (148.0 * per_sm)));
+          const double cycles = waves * 4000 + std::ceil(ctas / 148.0) * std::max(mma, copy) +
+                                (w + 3.0 * rows * cin * 2) / 48;
+          if (cycles < least) {
+            least = cycles;
+            best = t;
+          }
+        }
+      }
+  return least < 1e300;
+}
+
+inline bool wgrad_tile(int nx, int ny, int nz, int cin, int cout, WgradTile& t) {
+  const int blocks = (3 * cin + kTileM - 1) / kTileM;
+  // as many (dk, M block, channel) accumulators as tensor memory holds, and
+  // boxes of about 256 rows that fit the shared memory
+  bool found = false;
+  for (int ndk : {3, 1}) {
+    for (int mb = std::min(blocks, 4); mb >= 1 && !found; --mb)
+      for (int nt = std::min(cout, 128) / 16 * 16; nt >= 16 && !found; nt -= 16)
+        if (cout % nt == 0 && ndk * mb * nt <= 256) {
+          t.ndk = ndk;
+          t.mb = mb;
+          t.nt = nt;
+          found = true;
+        }
+    if (found) break;
+  }
+  if (!found) return false;
+  t.nmb = (blocks + t.mb - 1) / t.mb;
+  t.cols = tmem_columns(t.ndk * t.mb * t.nt);
+  for (int target : {512, 256, 128, 64, 32}) {
+    t.nzb = (nz + 61) / 62;
+    t.bz = (nz + t.nzb - 1) / t.nzb;
+    if (t.bz + 2 > target) {
+      t.nzb = (nz + target - 3) / (target - 2);
+      t.bz = (nz + t.nzb - 1) / t.nzb;
+    }
+    t.zp = t.bz + 2;
+    t.bj = std::max(1, std::min(ny, target / t.zp));
+    t.njb = (ny + t.bj - 1) / t.bj;
+    t.bj = (ny + t.njb - 1) / t.njb;
+    t.rows = (t.bj * t.zp + 15) & ~15;
+    t.items = nx * t.njb * t.nzb;
+    t.cs = chunk_stride((t.rows + 2) * 16);
+    t.ds = chunk_stride(t.rows * 16);
+    // the last M block's rows beyond 3 cin lie past the last chunk of x
+    t.doff = (kGuard + t.mb * (kTileM / 8) * t.cs + 127) & ~127;
+    const int used = t.doff + (t.nt / 8) * t.ds + 128;
+    if (used > 100 * 1024 && target > 32) continue;
+    if (used > kMaxSmem) return false;
+    t.smem = smem_for(used, t.cols);
+    // large boxes only while every SM still gets work
+    if (t.items * 3 * (3 / t.ndk) * t.nmb * (cout / t.nt) >= 2 * 148 || target == 64 || target == 32) return true;
+  }
+  return true;
 }
 
 }  // namespace conv

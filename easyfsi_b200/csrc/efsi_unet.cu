@@ -79,33 +79,45 @@ struct Dims {
 
 __host__ __device__ inline Dims coarse_of(Dims d) { return Dims{(d.nx + 1) / 2, (d.ny + 1) / 2, (d.nz + 1) / 2}; }
 
-__device__ __forceinline__ int64_t parent_of(const Dims& f, const Dims& c, int64_t v) {
-  const int k = (int)(v % f.nz);
-  const int64_t ij = v / f.nz;
-  const int j = (int)(ij % f.ny), i = (int)(ij / f.ny);
-  return ((int64_t)(i >> 1) * c.ny + (j >> 1)) * c.nz + (k >> 1);
+// 8 consecutive channels of one voxel
+struct Ch8 {
+  __align__(16) bf16 v[8];
+};
+__device__ __forceinline__ Ch8 load8(const bf16* p) {
+  Ch8 c;
+  *reinterpret_cast<uint4*>(c.v) = __ldg(reinterpret_cast<const uint4*>(p));
+  return c;
+}
+__device__ __forceinline__ void store8(bf16* p, const Ch8& c) {
+  *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(c.v);
 }
 
-// average over the existing children of each coarse voxel
+// average over the existing children of each coarse voxel; a thread takes 8
+// channels (one 16-byte load per child)
 __global__ void k_pool(Dims f, Dims c, int ch, const bf16* __restrict__ x, bf16* __restrict__ y) {
-  UNET_STRIDE(q, c.n() * ch) {
-    const int cc = (int)(q % ch);
-    const int64_t v = q / ch;
+  const int oct = ch / 8;
+  UNET_STRIDE(q, c.n() * oct) {
+    const int cc = (int)(q % oct) * 8;
+    const int64_t v = q / oct;
     const int k = (int)(v % c.nz);
     const int64_t ij = v / c.nz;
     const int j = (int)(ij % c.ny), i = (int)(ij / c.ny);
-    float s = 0.0f;
+    float s[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
     int cnt = 0;
-    for (int a = 0; a < 2; ++a)
-      for (int b = 0; b < 2; ++b)
-        for (int d = 0; d < 2; ++d) {
-          const int fi = 2 * i + a, fj = 2 * j + b, fk = 2 * k + d;
-          if (fi < f.nx && fj < f.ny && fk < f.nz) {
-            s += __bfloat162float(x[(((int64_t)fi * f.ny + fj) * f.nz + fk) * ch + cc]);
-            ++cnt;
-          }
-        }
-    y[q] = __float2bfloat16_rn(s / (float)cnt);
+#pragma unroll
+    for (int o = 0; o < 8; ++o) {
+      const int fi = 2 * i + (o >> 2), fj = 2 * j + ((o >> 1) & 1), fk = 2 * k + (o & 1);
+      if (fi < f.nx && fj < f.ny && fk < f.nz) {
+        const Ch8 a = load8(x + (((int64_t)fi * f.ny + fj) * f.nz + fk) * ch + cc);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[e] += __bfloat162float(a.v[e]);
+        ++cnt;
+      }
+    }
+    Ch8 r;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) r.v[e] = __float2bfloat16_rn(s[e] / (float)cnt);
+    store8(y + v * ch + cc, r);
   }
 }
 
@@ -123,126 +135,83 @@ __global__ void k_pool_back(Dims f, Dims c, int ch, const float* __restrict__ gc
   }
 }
 
-// out[v] = [coarse[parent(v)] (ca channels), skip[v] (cb channels)]
-__global__ void k_up_concat(Dims f, Dims c, int ca, int cb, const bf16* __restrict__ coarse,
-                            const bf16* __restrict__ skip, bf16* __restrict__ out) {
-  const int co = ca + cb;
-  UNET_STRIDE(q, f.n() * co) {
-    const int cc = (int)(q % co);
-    const int64_t v = q / co;
-    out[q] = cc < ca ? coarse[parent_of(f, c, v) * ca + cc] : skip[v * cb + (cc - ca)];
-  }
-}
-
-// adjoint of k_up_concat: the first ca channels are summed over the children
-// into the coarse gradient (written), the last cb added into the skip gradient
+// adjoint of the decoder's input [up(coarse), skip]: the first ca channels are
+// summed over the children into the coarse gradient (written), the last cb
+// added into the skip gradient; a thread takes 4 channels
 __global__ void k_up_concat_back_coarse(Dims f, Dims c, int ca, int cb, const float* __restrict__ g,
                                         float* __restrict__ gcoarse) {
-  const int co = ca + cb;
-  UNET_STRIDE(q, c.n() * ca) {
-    const int cc = (int)(q % ca);
-    const int64_t v = q / ca;
+  const int co = ca + cb, quads = ca / 4;
+  UNET_STRIDE(q, c.n() * quads) {
+    const int cc = (int)(q % quads) * 4;
+    const int64_t v = q / quads;
     const int k = (int)(v % c.nz);
     const int64_t ij = v / c.nz;
     const int j = (int)(ij % c.ny), i = (int)(ij / c.ny);
-    float s = 0.0f;
-    for (int a = 0; a < 2; ++a)
-      for (int b = 0; b < 2; ++b)
-        for (int d = 0; d < 2; ++d) {
-          const int fi = 2 * i + a, fj = 2 * j + b, fk = 2 * k + d;
-          if (fi < f.nx && fj < f.ny && fk < f.nz) s += g[(((int64_t)fi * f.ny + fj) * f.nz + fk) * co + cc];
-        }
-    gcoarse[q] = s;
+    float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int o = 0; o < 8; ++o) {
+      const int fi = 2 * i + (o >> 2), fj = 2 * j + ((o >> 1) & 1), fk = 2 * k + (o & 1);
+      if (fi < f.nx && fj < f.ny && fk < f.nz) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(g + (((int64_t)fi * f.ny + fj) * f.nz + fk) * co + cc));
+        s.x += a.x;
+        s.y += a.y;
+        s.z += a.z;
+        s.w += a.w;
+      }
+    }
+    *reinterpret_cast<float4*>(gcoarse + v * ca + cc) = s;
   }
 }
 
 __global__ void k_up_concat_back_skip(Dims f, int ca, int cb, const float* __restrict__ g, float* __restrict__ gskip) {
-  const int co = ca + cb;
-  UNET_STRIDE(q, f.n() * cb) {
-    const int cc = (int)(q % cb);
-    const int64_t v = q / cb;
-    gskip[q] += g[v * co + ca + cc];
+  const int co = ca + cb, quads = cb / 4;
+  UNET_STRIDE(q, f.n() * quads) {
+    const int cc = (int)(q % quads) * 4;
+    const int64_t v = q / quads;
+    const float4 a = __ldg(reinterpret_cast<const float4*>(g + v * co + ca + cc));
+    float4* d = reinterpret_cast<float4*>(gskip + v * cb + cc);
+    float4 r = *d;
+    r.x += a.x;
+    r.y += a.y;
+    r.z += a.z;
+    r.w += a.w;
+    *d = r;
   }
 }
 
-// dpre = relu ? dy * (y > 0) : dy, as BF16; bias gradient summed per block
+// dpre = relu ? dy * (y > 0) : dy, as BF16, and the bias gradient.  A thread
+// takes 8 channels, the same ones in every turn (the launch's grid is a
+// multiple of 3, so its stride is one of every channel count's octets), and
+// keeps their sums in registers until the end.
 __global__ void k_relu_back(int64_t n, int ch, int relu, const float* __restrict__ dy, const bf16* __restrict__ y,
                             bf16* __restrict__ dpre, float* __restrict__ dbias) {
   __shared__ float sb[128];
   for (int c = threadIdx.x; c < ch; c += blockDim.x) sb[c] = 0.0f;
   __syncthreads();
-  UNET_STRIDE(q, n * ch) {
-    float g = dy[q];
-    if (relu && !(__bfloat162float(y[q]) > 0.0f)) g = 0.0f;
-    const bf16 gb = __float2bfloat16_rn(g);
-    dpre[q] = gb;
-    const float gr = __bfloat162float(gb);
-    if (gr != 0.0f) atomicAdd(&sb[q % ch], gr);
+  const int oct = ch / 8;
+  float sum[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+  int c0 = -1;
+  UNET_STRIDE(q, n * oct) {
+    c0 = (int)(q % oct) * 8;
+    const float4 a = __ldg(reinterpret_cast<const float4*>(dy + 8 * q)),
+                 b = __ldg(reinterpret_cast<const float4*>(dy + 8 * q + 4));
+    const float g[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    Ch8 out, act;
+    if (relu) act = load8(y + 8 * q);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      out.v[e] = __float2bfloat16_rn(relu && !(__bfloat162float(act.v[e]) > 0.0f) ? 0.0f : g[e]);
+      sum[e] += __bfloat162float(out.v[e]);
+    }
+    store8(dpre + 8 * q, out);
+  }
+  if (c0 >= 0) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) atomicAdd(&sb[c0 + e], sum[e]);
   }
   __syncthreads();
   for (int c = threadIdx.x; c < ch; c += blockDim.x)
     if (sb[c] != 0.0f) atomicAdd(dbias + c, sb[c]);
-}
-
-// Weight gradient on the CUDA cores: dW[co][t][ci] += sum_v dpre[v][co] X[v + off(t)][ci]
-// over this block's voxel chunk, staged 32 voxels at a time in shared memory.
-constexpr int kWgThreads = 256;
-constexpr int kWgChunk = 2048;
-constexpr int kWgSub = 32;
-
-__global__ void __launch_bounds__(kWgThreads) k_wgrad(Dims d, int cin, int cout, const bf16* __restrict__ x,
-                                                      const bf16* __restrict__ dpre, float* __restrict__ dw) {
-  extern __shared__ float wg_smem[];
-  float* sg = wg_smem;                  // [kWgSub][cout]
-  float* sx = wg_smem + kWgSub * cout;  // [kWgSub][cin]
-  const int t = blockIdx.y;
-  const int di = t / 9 - 1, dj = (t / 3) % 3 - 1, dk = t % 3 - 1;
-  const int64_t n = d.n();
-  const int64_t vbeg = (int64_t)blockIdx.x * kWgChunk, vend = min(n, vbeg + kWgChunk);
-  const int nout = cout * cin;
-  constexpr int kPer = 28;  // outputs per thread (cout * cin <= 256 * 28)
-  float acc[kPer];
-#pragma unroll
-  for (int q = 0; q < kPer; ++q) acc[q] = 0.0f;
-  for (int64_t s0 = vbeg; s0 < vend; s0 += kWgSub) {
-    __syncthreads();
-    for (int q = threadIdx.x; q < kWgSub * cout; q += kWgThreads) {
-      const int r = q / cout, c = q - r * cout;
-      const int64_t v = s0 + r;
-      sg[q] = v < vend ? __bfloat162float(dpre[v * cout + c]) : 0.0f;
-    }
-    for (int q = threadIdx.x; q < kWgSub * cin; q += kWgThreads) {
-      const int r = q / cin, c = q - r * cin;
-      const int64_t v = s0 + r;
-      float val = 0.0f;
-      if (v < vend) {
-        const int k = (int)(v % d.nz);
-        const int64_t ij = v / d.nz;
-        const int j = (int)(ij % d.ny), i = (int)(ij / d.ny);
-        const int ii = i + di, jj = j + dj, kk = k + dk;
-        if (ii >= 0 && ii < d.nx && jj >= 0 && jj < d.ny && kk >= 0 && kk < d.nz)
-          val = __bfloat162float(x[(((int64_t)ii * d.ny + jj) * d.nz + kk) * cin + c]);
-      }
-      sx[q] = val;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < kPer; ++q) {
-      const int o = threadIdx.x + q * kWgThreads;
-      if (o >= nout) break;
-      const int co = o / cin, ci = o - co * cin;
-      float a = acc[q];
-      for (int r = 0; r < kWgSub; ++r) a += sg[r * cout + co] * sx[r * cin + ci];
-      acc[q] = a;
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < kPer; ++q) {
-    const int o = threadIdx.x + q * kWgThreads;
-    if (o >= nout) break;
-    const int co = o / cin, ci = o - co * cin;
-    if (acc[q] != 0.0f) atomicAdd(dw + ((int64_t)co * 27 + t) * cin + ci, acc[q]);
-  }
 }
 
 // BF16 copy of the FP32 master weights, and the flipped / transposed copy for
@@ -293,6 +262,10 @@ __global__ void k_loss(int64_t n, const float* __restrict__ out, const float* __
 
 #undef UNET_STRIDE
 
+unsigned relu_grid(int64_t octets) {
+  return 3u * (unsigned)std::max<int64_t>(1, std::min<int64_t>((octets + 767) / 768, 148));
+}
+
 unsigned grid_for(int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 148 * 32)); }
 
 }  // namespace
@@ -304,19 +277,19 @@ using namespace efsi;
 // The network object
 // ---------------------------------------------------------------------------
 namespace efsi {
-// Buffers of one volume size: layer outputs, decoder inputs, pooled inputs,
+// Buffers of one volume size: layer outputs, pooled inputs,
 // the FP32 output and the backward pass's gradients.
 struct UnetWorkspace {
   Dims dims[kLevels] = {};
   bf16* act[kLayers] = {};     // layer outputs
-  bf16* cat[3] = {};           // decoder inputs [up, skip] at levels 2, 1, 0
   bf16* pooled[3] = {};        // encoder inputs at levels 1, 2, 3
   float* outf = nullptr;       // FP32 output of the last layer
   float* gbuf[2] = {};         // gradient ping-pong (FP32), sized for the largest layer input
   float* gskip[kLevels] = {};  // accumulated gradients of e_0 .. e_3
-  float* gcoarse = nullptr;
   bf16* dpre = nullptr;
   float* dout = nullptr;
+  conv::ConvTile fwd[kLayers], bwd[kLayers];  // boxes of the layers' convolutions and input gradients
+  conv::WgradTile wg[kLayers];                // and weight gradients
 };
 }  // namespace efsi
 
@@ -349,15 +322,13 @@ constexpr int kMaxWorkspaces = 8;
 
 void free_workspace(UnetWorkspace* W) {
   for (auto& a : W->act) cudaFree(a), a = nullptr;
-  for (auto& a : W->cat) cudaFree(a), a = nullptr;
   for (auto& a : W->pooled) cudaFree(a), a = nullptr;
   for (auto& a : W->gbuf) cudaFree(a), a = nullptr;
   for (auto& a : W->gskip) cudaFree(a), a = nullptr;
   cudaFree(W->outf);
-  cudaFree(W->gcoarse);
   cudaFree(W->dpre);
   cudaFree(W->dout);
-  W->outf = W->gcoarse = W->dout = nullptr;
+  W->outf = W->dout = nullptr;
   W->dpre = nullptr;
 }
 
@@ -376,6 +347,17 @@ int ensure_workspace(efsi_unet* U, int nx, int ny, int nz) {
   const Dims d0{nx, ny, nz};
   W->dims[0] = d0;
   for (int l = 1; l < kLevels; ++l) W->dims[l] = coarse_of(W->dims[l - 1]);
+  for (int l = 0; l < kLayers; ++l) {
+    const LayerSpec& L = kSpec[l];
+    const Dims& d = W->dims[L.level];
+    if (!conv::conv_tile(d.nx, d.ny, d.nz, L.cin, L.cout, W->fwd[l]) ||
+        !conv::conv_tile(d.nx, d.ny, d.nz, L.cout, L.cin, W->bwd[l]) ||
+        !conv::wgrad_tile(d.nx, d.ny, d.nz, L.cin, L.cout, W->wg[l])) {
+      delete W;
+      set_error("no convolution box fits the shared memory");
+      return EFSI_ERR_ARG;
+    }
+  }
   auto alloc_bf = [](bf16** p, int64_t n) { return cudaMalloc(p, (size_t)std::max<int64_t>(n, 1) * sizeof(bf16)); };
   auto alloc_f = [](float** p, int64_t n) { return cudaMalloc(p, (size_t)std::max<int64_t>(n, 1) * sizeof(float)); };
   int64_t gmax = 0;
@@ -385,15 +367,12 @@ int ensure_workspace(efsi_unet* U, int nx, int ny, int nz) {
     gmax = std::max(gmax, n * std::max(kSpec[l].cin, kSpec[l].cout));
   }
   for (int q = 0; q < 3; ++q) {
-    const int l = 2 - q;  // decoder levels 2, 1, 0
-    const int64_t n = W->dims[l].n();
-    if (alloc_bf(&W->cat[q], n * (kCh[l + 1] + kCh[l])) != cudaSuccess) goto fail;
     if (alloc_bf(&W->pooled[q], W->dims[q + 1].n() * kCh[q]) != cudaSuccess) goto fail;
   }
   for (int l = 0; l < kLevels; ++l)
     if (alloc_f(&W->gskip[l], W->dims[l].n() * kCh[l]) != cudaSuccess) goto fail;
   if (alloc_f(&W->gbuf[0], gmax) != cudaSuccess || alloc_f(&W->gbuf[1], gmax) != cudaSuccess ||
-      alloc_f(&W->gcoarse, gmax) != cudaSuccess || alloc_bf(&W->dpre, gmax) != cudaSuccess ||
+      alloc_bf(&W->dpre, gmax) != cudaSuccess ||
       alloc_f(&W->outf, d0.n() * kOutCh) != cudaSuccess || alloc_f(&W->dout, d0.n() * kOutCh) != cudaSuccess)
     goto fail;
   U->spaces.push_back(W);
@@ -411,30 +390,31 @@ fail:
 int set_kernel_attributes() {
   static bool done = false;
   if (done) return EFSI_OK;
-  EFSI_CUDA_CHECK(cudaFuncSetAttribute(conv::k_conv3d_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-  EFSI_CUDA_CHECK(cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
+  EFSI_CUDA_CHECK(
+      cudaFuncSetAttribute(conv::k_conv3d_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, conv::kMaxSmem));
+  EFSI_CUDA_CHECK(
+      cudaFuncSetAttribute(conv::k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, conv::kMaxSmem));
   done = true;
   return EFSI_OK;
 }
 
-int conv_launch(const Dims& d, int cin, int cout, const bf16* x, const bf16* w, const float* bias, int relu, bf16* y,
-                float* yf, int* error, cudaStream_t s) {
-  conv::ConvArgs A{d.nx, d.ny, d.nz, cin, cout, x, w, bias, relu, y, yf, error};
-  // enough shared memory per CTA that the CTAs resident on an SM never ask for
-  // more than its 512 tensor-memory columns
-  const int per_sm = 512 / (int)conv::tmem_columns(cout);
-  const int smem = std::max(conv::conv_smem_bytes(cin, cout), 228 * 1024 / per_sm + 1024);
+int conv_launch(const conv::ConvTile& T, const Dims& d, int cin, int cout, const conv::ConvInput& in, const bf16* w,
+                const float* bias, int relu, bf16* y, float* yf, int* error, cudaStream_t s) {
+  conv::ConvArgs A{d.nx, d.ny, d.nz, cin, cout, in, w, bias, relu, y, yf, error};
   EFSI_TRY(set_kernel_attributes());
-  const unsigned blocks = (unsigned)((d.n() + conv::kTileM - 1) / conv::kTileM);
-  EFSI_COUNTED conv::k_conv3d_tc<<<blocks, conv::kThreads, smem, s>>>(A);
+  const dim3 grid((unsigned)(T.nzb * T.njb * T.nib), (unsigned)(cout / T.nt));
+  EFSI_COUNTED conv::k_conv3d_tc<<<grid, conv::kThreads, T.smem, s>>>(A, T);
   return EFSI_OK;
 }
 
-int wgrad_launch(const Dims& d, int cin, int cout, const bf16* x, const bf16* dpre, float* dw, cudaStream_t s) {
+int wgrad_launch(const conv::WgradTile& T, const Dims& d, int cin, int cout, const conv::ConvInput& in,
+                 const bf16* dpre, float* dw, int* error, cudaStream_t s) {
   EFSI_TRY(set_kernel_attributes());
-  const dim3 grid((unsigned)((d.n() + kWgChunk - 1) / kWgChunk), 27);
-  const int smem = kWgSub * (cin + cout) * (int)sizeof(float);
-  EFSI_COUNTED k_wgrad<<<grid, kWgThreads, smem, s>>>(d, cin, cout, x, dpre, dw);
+  conv::WgradArgs A{d.nx, d.ny, d.nz, cin, cout, in, dpre, dw, error};
+  const unsigned gy = 3u * (unsigned)(3 / T.ndk), gz = (unsigned)(T.nmb * (cout / T.nt));
+  // two CTAs per SM take the boxes in turn; each adds its sums once
+  const unsigned gx = (unsigned)std::min<int64_t>(T.items, std::max<int64_t>(1, 2 * 148 / (int64_t)(gy * gz)));
+  EFSI_COUNTED conv::k_wgrad_tc<<<dim3(gx, gy, gz), conv::kThreads, T.smem, s>>>(A, T);
   return EFSI_OK;
 }
 
@@ -448,51 +428,41 @@ int refresh_bf16(efsi_unet* U, cudaStream_t s) {
   return EFSI_OK;
 }
 
+// Input of layer l during the forward pass: the first layer of a decoder
+// block reads the coarser level's output (upsampled) and the encoder's.
+conv::ConvInput layer_input(efsi_unet* U, const bf16* input, int l) {
+  bf16* const* act = U->w->act;
+  if (l == 0) return {input, nullptr, 0};
+  if (l < 8) return {(l % 2 == 1) ? act[l - 1] : U->w->pooled[l / 2 - 1], nullptr, 0};
+  if (l < 14 && l % 2 == 0) {
+    const int lv = kSpec[l].level;
+    return {act[2 * lv + 1], act[l - 1], kCh[lv + 1]};
+  }
+  return {act[l - 1], nullptr, 0};
+}
+
 // Forward pass over the workspace volume; input [n0][16] BF16.
 int forward(efsi_unet* U, const bf16* input, cudaStream_t s) {
-  const bf16* x = input;
   int* err = U->run_error != nullptr ? U->run_error : U->error;
+  auto run = [&](int l, float* outf) {
+    const LayerSpec& L = kSpec[l];
+    return conv_launch(U->w->fwd[l], U->w->dims[L.level], L.cin, L.cout, layer_input(U, input, l), U->wb[l],
+                       U->p + U->boff[l], L.relu, U->w->act[l], outf, err, s);
+  };
   // encoder
   for (int l = 0; l < kLevels; ++l) {
     const Dims& d = U->w->dims[l];
-    if (l > 0) {
-      EFSI_COUNTED k_pool<<<grid_for(d.n() * kCh[l - 1]), 256, 0, s>>>(U->w->dims[l - 1], d, kCh[l - 1], U->w->act[2 * l - 1],
-                                                                    U->w->pooled[l - 1]);
-      x = U->w->pooled[l - 1];
-    }
-    const int a = 2 * l, b = 2 * l + 1;
-    EFSI_TRY(conv_launch(d, kSpec[a].cin, kSpec[a].cout, x, U->wb[a], U->p + U->boff[a], 1, U->w->act[a], nullptr,
-                         err, s));
-    EFSI_TRY(conv_launch(d, kSpec[b].cin, kSpec[b].cout, U->w->act[a], U->wb[b], U->p + U->boff[b], 1, U->w->act[b],
-                         nullptr, err, s));
+    if (l > 0)
+      EFSI_COUNTED k_pool<<<grid_for(d.n() * kCh[l - 1] / 8), 256, 0, s>>>(U->w->dims[l - 1], d, kCh[l - 1],
+                                                                        U->w->act[2 * l - 1], U->w->pooled[l - 1]);
+    EFSI_TRY(run(2 * l, nullptr));
+    EFSI_TRY(run(2 * l + 1, nullptr));
   }
-  // decoder
-  const bf16* coarse = U->w->act[7];
-  for (int q = 0; q < 3; ++q) {
-    const int l = 2 - q;
-    const Dims& d = U->w->dims[l];
-    const int ca = kCh[l + 1];
-    EFSI_COUNTED k_up_concat<<<grid_for(d.n() * (ca + kCh[l])), 256, 0, s>>>(d, U->w->dims[l + 1], ca, kCh[l], coarse,
-                                                                          U->w->act[2 * l + 1], U->w->cat[q]);
-    const int a = 8 + 2 * q, b = 9 + 2 * q;
-    EFSI_TRY(conv_launch(d, kSpec[a].cin, kSpec[a].cout, U->w->cat[q], U->wb[a], U->p + U->boff[a], 1, U->w->act[a],
-                         nullptr, err, s));
-    EFSI_TRY(conv_launch(d, kSpec[b].cin, kSpec[b].cout, U->w->act[a], U->wb[b], U->p + U->boff[b], 1, U->w->act[b],
-                         nullptr, err, s));
-    coarse = U->w->act[b];
-  }
-  EFSI_TRY(conv_launch(U->w->dims[0], kSpec[14].cin, kSpec[14].cout, U->w->act[13], U->wb[14], U->p + U->boff[14], 0,
-                       U->w->act[14], U->w->outf, err, s));
+  // decoder and output
+  for (int l = 8; l < 14; ++l) EFSI_TRY(run(l, nullptr));
+  EFSI_TRY(run(14, U->w->outf));
   EFSI_LAUNCH_CHECK();
   return EFSI_OK;
-}
-
-// Input of layer l during the forward pass.
-const bf16* layer_input(efsi_unet* U, const bf16* input, int l) {
-  if (l == 0) return input;
-  if (l < 8) return (l % 2 == 1) ? U->w->act[l - 1] : U->w->pooled[l / 2 - 1];
-  if (l < 14) return (l % 2 == 0) ? U->w->cat[(l - 8) / 2] : U->w->act[l - 1];
-  return U->w->act[13];
 }
 
 // Backward of one layer: gy (FP32 [n][cout]) -> parameter gradients, and the
@@ -501,11 +471,13 @@ int layer_backward(efsi_unet* U, const bf16* input, int l, const float* gy, floa
   const LayerSpec& L = kSpec[l];
   const Dims& d = U->w->dims[L.level];
   const int64_t n = d.n();
-  EFSI_COUNTED k_relu_back<<<grid_for(n * L.cout), 256, 0, s>>>(n, L.cout, L.relu, gy, U->w->act[l], U->w->dpre,
-                                                             U->g + U->boff[l]);
-  EFSI_TRY(wgrad_launch(d, L.cin, L.cout, layer_input(U, input, l), U->w->dpre, U->g + U->woff[l], s));
+  EFSI_COUNTED k_relu_back<<<relu_grid(n * L.cout / 8), 256, 0, s>>>(n, L.cout, L.relu, gy, U->w->act[l], U->w->dpre,
+                                                                  U->g + U->boff[l]);
+  EFSI_TRY(wgrad_launch(U->w->wg[l], d, L.cin, L.cout, layer_input(U, input, l), U->w->dpre, U->g + U->woff[l],
+                        U->error, s));
   if (gx != nullptr)
-    EFSI_TRY(conv_launch(d, L.cout, L.cin, U->w->dpre, U->wt[l], nullptr, 0, nullptr, gx, U->error, s));
+    EFSI_TRY(conv_launch(U->w->bwd[l], d, L.cout, L.cin, {U->w->dpre, nullptr, 0}, U->wt[l], nullptr, 0, nullptr, gx,
+                         U->error, s));
   EFSI_LAUNCH_CHECK();
   return EFSI_OK;
 }
@@ -527,14 +499,12 @@ int backward(efsi_unet* U, const bf16* input, const float* dout, cudaStream_t s)
     float* t2 = (t1 == ga) ? gb : ga;
     EFSI_TRY(layer_backward(U, input, a, t1, t2, s));  // -> g([up, skip])
     const int ca = kCh[l + 1], cb = kCh[l];
-    EFSI_COUNTED k_up_concat_back_skip<<<grid_for(U->w->dims[l].n() * cb), 256, 0, s>>>(U->w->dims[l], ca, cb, t2,
-                                                                                   U->w->gskip[l]);
-    EFSI_COUNTED k_up_concat_back_coarse<<<grid_for(U->w->dims[l + 1].n() * ca), 256, 0, s>>>(
-        U->w->dims[l], U->w->dims[l + 1], ca, cb, t2, U->w->gcoarse);
+    EFSI_COUNTED k_up_concat_back_skip<<<grid_for(U->w->dims[l].n() * cb / 4), 256, 0, s>>>(U->w->dims[l], ca, cb, t2,
+                                                                                       U->w->gskip[l]);
     // the coarse gradient is that of d_{l+1} (or e_3 for the deepest block)
     float* nxt = (t2 == ga) ? gb : ga;
-    EFSI_CUDA_CHECK(cudaMemcpyAsync(nxt, U->w->gcoarse, (size_t)U->w->dims[l + 1].n() * ca * sizeof(float),
-                                    cudaMemcpyDeviceToDevice, s));
+    EFSI_COUNTED k_up_concat_back_coarse<<<grid_for(U->w->dims[l + 1].n() * ca / 4), 256, 0, s>>>(
+        U->w->dims[l], U->w->dims[l + 1], ca, cb, t2, nxt);
     gcur = nxt;
   }
   // gcur is g(e_3) from the decoder; the encoder from level 3 down to 0
@@ -600,9 +570,13 @@ int efsi_conv3d_bf16(int32_t nx, int32_t ny, int32_t nz, int32_t cin, int32_t co
   EFSI_ARG_CHECK(cout >= 16 && cout % 16 == 0 && cout <= 256, "cout must be a multiple of 16 in [16, 256]");
   EFSI_ARG_CHECK(x != nullptr && w != nullptr && error_device != nullptr && (y != nullptr || yf != nullptr),
                  "null argument");
-  EFSI_ARG_CHECK(conv::conv_smem_bytes(cin, cout) <= 200 * 1024, "cin x cout too large for the shared-memory stages");
-  EFSI_TRY(conv_launch(Dims{nx, ny, nz}, cin, cout, static_cast<const bf16*>(x), static_cast<const bf16*>(w), bias,
-                       relu, static_cast<bf16*>(y), yf, error_device, as_stream(stream)));
+  conv::ConvTile T;
+  EFSI_ARG_CHECK(8 * (int64_t)cin * (conv::kTileM + cout) + 128 <= 200 * 1024 &&
+                     conv::conv_tile(nx, ny, nz, cin, cout, T),
+                 "cin x cout too large for the shared memory");
+  EFSI_TRY(conv_launch(T, Dims{nx, ny, nz}, cin, cout, {static_cast<const bf16*>(x), nullptr, 0},
+                       static_cast<const bf16*>(w), bias, relu, static_cast<bf16*>(y), yf, error_device,
+                       as_stream(stream)));
   EFSI_LAUNCH_CHECK();
   return EFSI_OK;
 }
@@ -613,8 +587,10 @@ int efsi_conv3d_wgrad(int32_t nx, int32_t ny, int32_t nz, int32_t cin, int32_t c
   EFSI_ARG_CHECK(cin >= 16 && cin % 16 == 0 && cout >= 16 && cout % 16 == 0 && cin * cout <= 256 * 28,
                  "unsupported channel counts for the weight gradient");
   EFSI_ARG_CHECK(x != nullptr && dy != nullptr && dw != nullptr, "null argument");
-  EFSI_TRY(wgrad_launch(Dims{nx, ny, nz}, cin, cout, static_cast<const bf16*>(x), static_cast<const bf16*>(dy), dw,
-                        as_stream(stream)));
+  conv::WgradTile T;
+  EFSI_ARG_CHECK(conv::wgrad_tile(nx, ny, nz, cin, cout, T), "unsupported channel counts for the weight gradient");
+  EFSI_TRY(wgrad_launch(T, Dims{nx, ny, nz}, cin, cout, {static_cast<const bf16*>(x), nullptr, 0},
+                        static_cast<const bf16*>(dy), dw, nullptr, as_stream(stream)));
   EFSI_LAUNCH_CHECK();
   return EFSI_OK;
 }

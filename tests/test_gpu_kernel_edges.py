@@ -1,8 +1,11 @@
 """Kernels at the sizes where their tiles, remainders and selection rules can
 go wrong, against the CPU oracle or a plain float64 restatement."""
 
+import math
+
 import numpy as np
 import pytest
+import torch
 
 from oracle import oracle as orc
 
@@ -131,3 +134,71 @@ def test_predictor_matches_the_oracle(nodes, graded, dt, rk2):
     fl.predict(dt, advection_scheme="rk2" if rk2 else "euler")
     ofl.predict(dt, rk2=rk2)
     assert _rel(fl.velocity.to_numpy(), ofl.velocity) <= 2.0**-24
+
+
+# ---------------------------------------------------------------------------
+# tensor-core convolution and weight gradient
+# ---------------------------------------------------------------------------
+
+
+def _volume(shape, ch, gen):
+    return torch.randn(shape + (ch,), generator=gen, device="cuda").to(torch.bfloat16)
+
+
+def _shifted(x, t):
+    """x[v + off(t)], zeros outside the volume (float64)."""
+    p = torch.nn.functional.pad(x, (0, 0, 1, 1, 1, 1, 1, 1))
+    i, j, k = t // 9, (t // 3) % 3, t % 3
+    return p[i : i + x.shape[0], j : j + x.shape[1], k : k + x.shape[2]]
+
+
+CONV_SHAPES = [
+    (16, 16, (1, 1, 1)), (16, 16, (2, 1, 62)), (16, 32, (3, 5, 63)), (48, 16, (17, 9, 65)), (16, 48, (5, 33, 130)),
+    (64, 64, (4, 4, 4)), (112, 48, (3, 9, 34)), (48, 112, (2, 7, 16)), (176, 16, (3, 3, 64)), (64, 256, (2, 3, 5)),
+    (80, 32, (20, 18, 32)),
+]
+
+
+@pytest.mark.parametrize("cin,cout,shape", CONV_SHAPES)
+def test_convolution_boxes(cin, cout, shape):
+    """Every box rule: lines split along z, several MMA tiles per plane, plane
+    rings, channel splits, single lines.  FP32 sums of 27 cin products against
+    float64 on the same BF16 values."""
+    from easyfsi_b200 import _native
+
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(cin * 1000 + cout)
+    x = _volume(shape, cin, gen)
+    w = (torch.randn((cout, 27, cin), generator=gen, device="cuda") / math.sqrt(27 * cin)).to(torch.bfloat16)
+    b = torch.randn(cout, generator=gen, device="cuda")
+    yf = torch.full(shape + (cout,), float("nan"), dtype=torch.float32, device="cuda")
+    yb = torch.zeros(shape + (cout,), dtype=torch.bfloat16, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _native.call("efsi_conv3d_bf16", *shape, cin, cout, x.data_ptr(), w.data_ptr(), b.data_ptr(), 1, yb.data_ptr(),
+                 yf.data_ptr(), err.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    xd, wd = x.double(), w.double()
+    ref = torch.relu(sum(_shifted(xd, t) @ wd[:, t].T for t in range(27)) + b.double())
+    assert _rel(yf.cpu().numpy(), ref.cpu().numpy()) <= 1e-5
+    assert torch.equal(yb, yf.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("cin,cout,shape", [c for c in CONV_SHAPES if c[0] * c[1] <= 7168] + [
+    (448, 16, (2, 2, 9)), (16, 448, (3, 4, 17)), (16, 16, (40, 33, 31))])
+def test_weight_gradient_boxes(cin, cout, shape):
+    """Boxes of a plane, several M blocks and channel splits; FP32 sums over
+    the voxels against float64, added to what is there."""
+    from easyfsi_b200 import _native
+
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(cin * 1000 + cout + 1)
+    x, g = _volume(shape, cin, gen), _volume(shape, cout, gen)
+    start = torch.randn((cout, 27, cin), generator=gen, device="cuda")
+    dw = start.clone()
+    _native.call("efsi_conv3d_wgrad", *shape, cin, cout, x.data_ptr(), g.data_ptr(), dw.data_ptr(),
+                 torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    xd, gd = x.double(), g.double().reshape(-1, cout)
+    ref = torch.stack([gd.T @ _shifted(xd, t).reshape(-1, cin) for t in range(27)], dim=1) + start.double()
+    assert _rel(dw.cpu().numpy(), ref.cpu().numpy()) <= 1e-5

@@ -42,6 +42,7 @@
 #include "efsi_unet_internal.cuh"
 #include <cuda_bf16.h>
 #include "efsi_march.cuh"
+#include "efsi_column.cuh"
 
 namespace efsi {
 
@@ -2026,6 +2027,23 @@ static void preload_kernels() {
 #undef EFSI_MIXED_FNS
   };
   for (const void* f : fns) cudaFuncGetAttributes(&a, f);
+#define EFSI_COLUMN_SWEEP(T, P, A, D) {(const void*)kc_sweep<T, P, A, D>, ColumnSweep<T, P, A, D>::Lay::kSmem}
+#define EFSI_COLUMN_FNS(A)                                                                                       \
+  EFSI_COLUMN_SWEEP(double, false, A, false), EFSI_COLUMN_SWEEP(double, false, A, true),                         \
+      EFSI_COLUMN_SWEEP(double, true, A, false), EFSI_COLUMN_SWEEP(double, true, A, true),                       \
+      EFSI_COLUMN_SWEEP(float, false, A, false), EFSI_COLUMN_SWEEP(float, false, A, true),                       \
+      EFSI_COLUMN_SWEEP(float, true, A, false), EFSI_COLUMN_SWEEP(float, true, A, true),                         \
+      {(const void*)kc_spmv_dir<true, A>, ColumnSpmv<true, A>::Lay::kSmem},                                      \
+      {(const void*)kc_spmv_dir<false, A>, ColumnSpmv<false, A>::Lay::kSmem},                                    \
+      {(const void*)kc_restrict<double, A>, ColumnRestrict<double, A>::Lay::kSmem},                              \
+      {(const void*)kc_restrict<float, A>, ColumnRestrict<float, A>::Lay::kSmem}
+  const std::pair<const void*, int> columns[] = {EFSI_COLUMN_FNS(false), EFSI_COLUMN_FNS(true)};
+#undef EFSI_COLUMN_FNS
+#undef EFSI_COLUMN_SWEEP
+  for (const auto& d : columns) {
+    cudaFuncGetAttributes(&a, d.first);
+    cudaFuncSetAttribute(d.first, cudaFuncAttributeMaxDynamicSharedMemorySize, d.second);
+  }
   // the plane-marching kernels take up to ~70 KB of dynamic shared memory
 #define EFSI_MARCH_SMEM(A)                                                                                        \
   {(const void*)km_sweep<double, true, false, A, false>, march_smem<double, 1, double, true>()},                  \
@@ -2328,6 +2346,16 @@ int efsi_fv_plan_create(const efsi_level_desc* levels, int32_t n_levels, int32_t
       const MarchCfg ms = march_cfg(B.nx, B.ny, B.nz, nsm * 2);
       B.spchunk = ms.chunk;
       B.spgrid = ms.grid;
+      // the column kernels take two cells per thread along k: levels of at
+      // least 40 cells there fill most of a 64-cell tile (at 64^3 a coupled
+      // step takes the same time either way, at 128 x 128 x 256 13% less)
+      B.column = l == 0 && B.march && B.nz >= 40 && std::getenv("EFSI_NO_COLUMN") == nullptr;
+      const MarchCfg mc4 = column_cfg(B.nx, B.ny, B.nz, nsm * 4);
+      B.cchunk = mc4.chunk;
+      B.cgrid = mc4.grid;
+      // up to five sums per block of any launch shape (the autotuner's too)
+      const size_t tiles = (size_t)((B.nz + kMK - 1) / kMK) * ((B.ny + kCJ - 1) / kCJ);
+      max_blocks = std::max<size_t>(max_blocks, 2 * tiles * (size_t)((B.nx + 1) / 2));
     }
     size_t ncoef = 2 * (size_t)(B.nx + B.ny + B.nz);
     if (cudaMalloc(&B.coef, ncoef * sizeof(double)) != cudaSuccess || cudaMalloc(&B.mask, B.n) != cudaSuccess) {
@@ -2626,7 +2654,17 @@ namespace efsi {
 // TMA descriptors of level fields for the plane-marching kernels
 // ---------------------------------------------------------------------------
 // MAP_VALUE32: an FP32 value tile on level 0 (the mixed-precision V-cycle)
-enum : int { MAP_VALUE = 0, MAP_RHS = 1, MAP_MASK = 2, MAP_VALUE32 = 3 };
+// MAP_C*: the same for the column-marching kernels' tiles (64 x 8)
+enum : int {
+  MAP_VALUE = 0,
+  MAP_RHS = 1,
+  MAP_MASK = 2,
+  MAP_VALUE32 = 3,
+  MAP_CVALUE = 4,
+  MAP_CRHS = 5,
+  MAP_CMASK = 6,
+  MAP_CVALUE32 = 7
+};
 
 static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
@@ -2653,17 +2691,19 @@ static const CUtensorMap* plane_map(efsi_fv_plan* P, int l, const void* ptr, int
   auto enc = tensor_map_encoder();
   if (enc == nullptr || ptr == nullptr || (reinterpret_cast<uintptr_t>(ptr) & 15u) != 0) return nullptr;
   const LevelBuf& B = P->lv[l];
-  const int es = kind == MAP_MASK ? 1 : (l == 0 && kind != MAP_VALUE32 ? 8 : 4);
+  const bool mask = kind == MAP_MASK || kind == MAP_CMASK, f32 = kind == MAP_VALUE32 || kind == MAP_CVALUE32;
+  const bool col = kind >= MAP_CVALUE, halo = kind == MAP_VALUE || kind == MAP_CVALUE || f32;
+  const int es = mask ? 1 : (l == 0 && !f32 ? 8 : 4);
   if (((size_t)B.nz * es) % 16 != 0) return nullptr;
-  const CUtensorMapDataType dt = kind == MAP_MASK ? CU_TENSOR_MAP_DATA_TYPE_UINT8
-                                 : es == 8        ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64
-                                                  : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+  const CUtensorMapDataType dt = mask      ? CU_TENSOR_MAP_DATA_TYPE_UINT8
+                                 : es == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64
+                                           : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
   const cuuint64_t dims[3] = {(cuuint64_t)B.nz, (cuuint64_t)B.ny, (cuuint64_t)B.nx};
   const cuuint64_t strides[2] = {(cuuint64_t)B.nz * es, (cuuint64_t)B.nz * B.ny * es};
-  cuuint32_t box[3] = {(cuuint32_t)kMK, (cuuint32_t)kMJ, 1u};
-  if (kind == MAP_VALUE || kind == MAP_VALUE32) {
-    box[0] = (cuuint32_t)(kMK + 2 * (16 / es));
-    box[1] = (cuuint32_t)(kMJ + 2);
+  cuuint32_t box[3] = {(cuuint32_t)(col ? kCK : kMK), (cuuint32_t)(col ? kCJ : kMJ), 1u};
+  if (halo) {
+    box[0] += (cuuint32_t)(2 * (16 / es));
+    box[1] += 2u;
   }
   const cuuint32_t estr[3] = {1u, 1u, 1u};
   PlaneMap pm;
@@ -2684,6 +2724,23 @@ static bool launch_march_spmv(efsi_fv_plan* P, const LevelDev& L, bool copy, con
                               double* d_new, double* Ad, int outlet, double* partials, CgScalars* sc,
                               cudaStream_t s) {
   const LevelBuf& B = P->lv[0];
+  if (B.column) {
+    const CUtensorMap* cz = plane_map(P, 0, z, MAP_CVALUE);
+    const CUtensorMap* cm = plane_map(P, 0, B.mask, MAP_CMASK);
+    const CUtensorMap* cd = copy ? cz : plane_map(P, 0, d_old, MAP_CVALUE);
+    if (cz && cm && cd) {
+      const bool aux = L.fw != nullptr || L.iface != nullptr;
+#define EFSI_COLUMN_SPMV(COPY, AUX)                                                                               \
+  EFSI_COUNTED launch_pdl(kc_spmv_dir<COPY, AUX>, B.cgrid, dim3(32, kCWarps), ColumnSpmv<COPY, AUX>::Lay::kSmem, s, \
+                          L, B.cchunk, *cz, *cd, *cm, d_new, Ad, outlet, partials, sc)
+      if (copy && aux) EFSI_COLUMN_SPMV(true, true);
+      else if (copy) EFSI_COLUMN_SPMV(true, false);
+      else if (aux) EFSI_COLUMN_SPMV(false, true);
+      else EFSI_COLUMN_SPMV(false, false);
+#undef EFSI_COLUMN_SPMV
+      return true;
+    }
+  }
   const CUtensorMap* mz = plane_map(P, 0, z, MAP_VALUE);
   const CUtensorMap* mm = plane_map(P, 0, B.mask, MAP_MASK);
   const CUtensorMap* md = copy ? mz : plane_map(P, 0, d_old, MAP_VALUE);
@@ -2706,6 +2763,39 @@ static bool launch_march_spmv(efsi_fv_plan* P, const LevelDev& L, bool copy, con
   return true;
 }
 
+// One level-0 sweep of the V-cycle with the column kernels (right-hand side
+// -r; dots_delta: the PCG's dots are finished in it, with the reciprocal
+// denominators when the iterate is f64); false when they do not apply.
+template <typename TV>
+static bool launch_column_sweep(efsi_fv_plan* P, const LevelDev& L, const TV* p, const double* r, TV* out,
+                                double* out64, int outlet, double om, ProlongSrc pr, double* partials,
+                                const double* dots_delta, cudaStream_t s) {
+  const LevelBuf& B = P->lv[0];
+  const bool dots = dots_delta != nullptr, pro = pr.pc != nullptr, aux = L.fw != nullptr || L.iface != nullptr;
+  const double* rden = P->rden_ok[outlet ? 1 : 0] ? P->rden[outlet ? 1 : 0] : nullptr;
+  if (!B.column || (dots && sizeof(TV) == 8 && rden == nullptr)) return false;
+  const CUtensorMap* mp = plane_map(P, 0, p, sizeof(TV) == 8 ? MAP_CVALUE : MAP_CVALUE32);
+  const CUtensorMap* mr = plane_map(P, 0, r, MAP_CRHS);
+  const CUtensorMap* mm = plane_map(P, 0, B.mask, MAP_CMASK);
+  const CUtensorMap* md = dots ? plane_map(P, 0, dots_delta, MAP_CRHS) : mr;
+  const CUtensorMap* mi = dots && sizeof(TV) == 8 ? plane_map(P, 0, rden, MAP_CRHS) : mr;
+  if (!mp || !mr || !mm || !md || !mi) return false;
+#define EFSI_COLUMN(PRO, AUX, DOTS)                                                                              \
+  EFSI_COUNTED launch_pdl(kc_sweep<TV, PRO, AUX, DOTS>, B.cgrid, dim3(32, kCWarps),                              \
+                          ColumnSweep<TV, PRO, AUX, DOTS>::Lay::kSmem, s, L, B.cchunk, *mp, *mr, *mm, *md, *mi,  \
+                          out, out64, outlet, om, pr, partials, P->sc)
+  if (pro && aux && dots) EFSI_COLUMN(true, true, true);
+  else if (pro && aux) EFSI_COLUMN(true, true, false);
+  else if (pro && dots) EFSI_COLUMN(true, false, true);
+  else if (pro) EFSI_COLUMN(true, false, false);
+  else if (aux && dots) EFSI_COLUMN(false, true, true);
+  else if (aux) EFSI_COLUMN(false, true, false);
+  else if (dots) EFSI_COLUMN(false, false, true);
+  else EFSI_COLUMN(false, false, false);
+#undef EFSI_COLUMN
+  return true;
+}
+
 // One sweep with the marching kernels; false when the fields cannot be
 // streamed with TMA (the caller then runs the per-cell kernel).
 template <typename TP, bool kNegR, bool kZero, bool kAux>
@@ -2724,6 +2814,11 @@ static bool launch_march_sweep(efsi_fv_plan* P, int l, const LevelDev& L, const 
     EFSI_COUNTED launch_pdl(km_sweep0<TP, kNegR, kAux>, sweep0_grid(B.nx, B.ny, B.nz), blk, 0, s, L, rhs, out, outlet, om,
                                                                                            partials, P->sc, rden);
     return true;
+  }
+  if constexpr (std::is_same<TP, double>::value && kNegR) {
+    if (l == 0 && launch_column_sweep<double>(P, L, p, static_cast<const double*>(rhs), out, nullptr, outlet, om, pr,
+                                              partials, dots_delta, s))
+      return true;
   }
   const CUtensorMap* mp = plane_map(P, l, p, MAP_VALUE);
   const CUtensorMap* mr = plane_map(P, l, rhs, MAP_RHS);
@@ -2771,6 +2866,7 @@ static bool launch_sweep32(efsi_fv_plan* P, const float* p, const double* r, flo
                            double om, ProlongSrc pr, double* partials, const double* dots_delta, cudaStream_t s) {
   LevelDev L = level_dev(P, 0);
   const LevelBuf& B = P->lv[0];
+  if (launch_column_sweep<float>(P, L, p, r, out, out64, outlet, om, pr, partials, dots_delta, s)) return true;
   const CUtensorMap* mp = plane_map(P, 0, p, MAP_VALUE32);
   const CUtensorMap* mr = plane_map(P, 0, r, MAP_RHS);
   const CUtensorMap* mm = plane_map(P, 0, B.mask, MAP_MASK);
@@ -2833,6 +2929,24 @@ static bool launch_restrict(efsi_fv_plan* P, int l, const TP* p, const void* rhs
   LevelDev L = level_dev(P, l);
   const LevelBuf& B = P->lv[l];
   const LevelBuf& C = P->lv[l + 1];
+  if constexpr (kNegR) {
+    if (l == 0 && B.column) {
+      const CUtensorMap* mp = plane_map(P, l, p, sizeof(TP) == 8 ? MAP_CVALUE : MAP_CVALUE32);
+      const CUtensorMap* mr = plane_map(P, l, rhs, MAP_CRHS);
+      const CUtensorMap* mm = plane_map(P, l, B.mask, MAP_CMASK);
+      if (mp && mr && mm) {
+        const LevelDev LC = level_dev(P, l + 1);
+        if (L.fw != nullptr || L.iface != nullptr)
+          EFSI_COUNTED launch_pdl(kc_restrict<TP, true>, B.cgrid, dim3(32, kCWarps), ColumnRestrict<TP, true>::Lay::kSmem,
+                                  s, L, B.cchunk, *mp, *mr, *mm, outlet, LC, C.rhs, czero, omega, P->sc);
+        else
+          EFSI_COUNTED launch_pdl(kc_restrict<TP, false>, B.cgrid, dim3(32, kCWarps),
+                                  ColumnRestrict<TP, false>::Lay::kSmem, s, L, B.cchunk, *mp, *mr, *mm, outlet, LC, C.rhs,
+                                  czero, omega, P->sc);
+        return czero != nullptr;
+      }
+    }
+  }
   if (B.march) {
     using TR = typename std::conditional<kNegR, double, TP>::type;
     const CUtensorMap* mp = plane_map(P, l, p, (l == 0 && sizeof(TP) == 4) ? MAP_VALUE32 : MAP_VALUE);
@@ -3962,8 +4076,9 @@ extern "C" {
 // two untimed ones -- on level 0 the PCG's direction SpMV and a whole V-cycle
 // with the dots fused in, on a coarse level its plain sweep and restriction
 // (the sweep alone on a coarsest level without a tail): the plane-marching kernels
-// with 3 (the default), 1, 2, 4 or 6 blocks' worth of planes per SM and, on
-// levels >= 1, the tiled / per-cell kernels.  A candidate replaces the best so
+// with 3 (the default), 1, 2, 4 or 6 blocks' worth of planes per SM (the
+// column kernels of level 0: 4, 2, 3, 6 or 8) and, on levels >= 1, the tiled /
+// per-cell kernels.  A candidate replaces the best so
 // far only when it is more than 3% faster.  Level 0 keeps the plane march
 // whenever it can run (the PCG's dots are fused into its last sweep).  Every
 // candidate computes the same rows; only the block partition of the z-mean /
@@ -3995,7 +4110,7 @@ int efsi_fv_autotune(efsi_fv_plan* P, int32_t reps, int32_t* choice, double* bes
     LevelBuf& B = P->lv[l];
     std::vector<int> cands;
     if (B.march_ok) {
-      cands = {3, 1, 2, 4, 6};
+      cands = B.column ? std::vector<int>{4, 2, 3, 6, 8} : std::vector<int>{3, 1, 2, 4, 6};
       if (l > 0) cands.push_back(0);
     } else {
       cands = {0};
@@ -4004,10 +4119,10 @@ int efsi_fv_autotune(efsi_fv_plan* P, int32_t reps, int32_t* choice, double* bes
       if (m == 0) {
         B.march = false;
       } else {
-        const MarchCfg mc = march_cfg(B.nx, B.ny, B.nz, nsm * m);
+        const MarchCfg mc = B.column ? column_cfg(B.nx, B.ny, B.nz, nsm * m) : march_cfg(B.nx, B.ny, B.nz, nsm * m);
         B.march = true;
-        B.mchunk = mc.chunk;
-        B.mgrid = mc.grid;
+        (B.column ? B.cchunk : B.mchunk) = mc.chunk;
+        (B.column ? B.cgrid : B.mgrid) = mc.grid;
       }
     };
     auto pair = [&]() {

@@ -224,6 +224,9 @@ struct LevelBuf {
   unsigned mgrid = 1;  // and grid size
   int spchunk = 2;      // the direction SpMV's (two blocks per SM)
   unsigned spgrid = 1;
+  bool column = false;  // level 0: the column-marching kernels run the V-cycle and the SpMV
+  int cchunk = 2;       // their planes per block
+  unsigned cgrid = 1;
 };
 
 }  // namespace efsi

@@ -837,9 +837,8 @@ __global__ void __launch_bounds__(kMK* kTY, 2)
 // kNegR = false> / k_sweep<float, false, true>: the neighbours are zero, so
 // ns = 0 and only the row's own denominator and rhs enter), evaluated by the
 // restriction that produced the row's rhs value v.
-__device__ __forceinline__ float coarse_zero_sweep(const LevelDev& C, int ci, int cj, int ck, int64_t cc, float v,
-                                                   int outlet, double omega) {
-  const unsigned m = __ldg(C.mask + cc);
+__device__ __forceinline__ float coarse_zero_sweep(const LevelDev& C, unsigned m, int ci, int cj, int ck, int64_t cc,
+                                                   float v, int outlet, double omega) {
   float res = 0.0f;
   if (!(m & M_SOLID)) {
     double ns, den;
@@ -959,7 +958,7 @@ struct RestrictOp {
       const int cj = cj0 + rem / kCK, ck = ck0 + rem % kCK;
       if (ci < cnx && cj < cny && ck < cnz) {
         const int64_t cc = cidx(ci, cj, ck, cny, cnz);
-        cpa[cc] = coarse_zero_sweep(C, ci, cj, ck, cc, crhs[cc], outlet, omega);
+        cpa[cc] = coarse_zero_sweep(C, __ldg(C.mask + cc), ci, cj, ck, cc, crhs[cc], outlet, omega);
       }
     }
   }

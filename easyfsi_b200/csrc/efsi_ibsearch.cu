@@ -40,6 +40,8 @@ struct efsi_ib_search_plan {
   int64_t claim_cap = 0;
   float4* rec = nullptr;  // per item: kRecQuads quads of precomputed geometry
   int64_t rec_cap = 0;
+  float4* grp = nullptr;
+  int64_t grp_cap = 0;
   uint32_t* far_nodes = nullptr;  // nodes whose far classification is still open, and their count
   int64_t far_cap = 0;
   unsigned* far_count = nullptr;
@@ -139,6 +141,7 @@ struct SearchArgs {
   const int32_t* offset;   // null: every node visits every item
   const int32_t* entries;
   const float4* rec;       // per item: kRecQuads quads (k_ibs_records)
+  const float4* grp;       // per kGroup items: kGrpQuads quads (k_ibs_groups)
   uint32_t* far_nodes;     // nodes left to k_ibs_far, and their count
   unsigned* far_count;
   // per-node fields (hibm_mpm.py:5418-5436) and the four report counts
@@ -232,6 +235,71 @@ __global__ void k_ibs_records(SearchArgs A, float4* rec) {
   r[1] = make_float4(n.x, n.y, n.z, slack);
   r[2] = make_float4(b.x, b.y, b.z, 0.0f);
   r[3] = make_float4(c.x, c.y, c.z, 0.0f);
+}
+
+// Bounds of kGroup consecutive items, for nodes far from all of them:
+//   q0 = (c, R)       no point of an item is farther than R from c
+//   q1 = (nlo, D)     the items' normals lie between nlo and nhi, and
+//   q2 = (nhi, -)     dot(c - a, n) + slack <= D for each of them, so
+//   dot(p - a, n) + slack <= sum_x max((p - c)_x nlo_x, (p - c)_x nhi_x) + D
+// both with the rounding at c in them.  Degenerate items are left out; an item
+// that has no bound of its own, or a coordinate that is not finite, opens the
+// group to every node.
+constexpr int kGroup = 8, kGrpQuads = 3;
+
+__global__ void k_ibs_groups(SearchArgs A, float4* grp) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  const int n = items(A);
+  if (g >= (n + kGroup - 1) / kGroup) return;
+  const float inf = __int_as_float(0x7f800000);
+  const int t1 = min(n, (g + 1) * kGroup), corners = A.tri_count > 0 ? 3 : 1;
+  F3 lo = f3(inf, inf, inf), hi = f3(-inf, -inf, -inf), nlo = lo, nhi = hi;
+  bool any = false, always = false;
+  for (int t = g * kGroup; t < t1; ++t) {
+    const float4* r = A.rec + (int64_t)kRecQuads * t;
+    if (__ldg(r).w < 0.0f) continue;  // degenerate
+    any = true;
+    const F3 nn = xyz(__ldg(r + 1));
+    float sum = abs1(nn) + __ldg(r).w + __ldg(r + 1).w;
+    nlo = f3(fminf(nlo.x, nn.x), fminf(nlo.y, nn.y), fminf(nlo.z, nn.z));
+    nhi = f3(fmaxf(nhi.x, nn.x), fmaxf(nhi.y, nn.y), fmaxf(nhi.z, nn.z));
+    for (int v = 0; v < corners; ++v) {
+      const F3 x = xyz(__ldg(r + (v == 0 ? 0 : v + 1)));
+      sum += abs1(x);
+      lo = f3(fminf(lo.x, x.x), fminf(lo.y, x.y), fminf(lo.z, x.z));
+      hi = f3(fmaxf(hi.x, x.x), fmaxf(hi.y, x.y), fmaxf(hi.z, x.z));
+    }
+    // not finite, or its square would not be; a marker's normal far from unit length
+    if (!(sum < 1.0e18f) || abs1(nn) > 64.0f) always = true;
+  }
+  F3 c = f3(0.0f, 0.0f, 0.0f);
+  float R = -inf, D = -inf;
+  if (any && !always) {
+    c = scale(add(lo, hi), 0.5f);
+    const float at_c = 2.0f * kSlack * abs1(c);
+    for (int t = g * kGroup; t < t1; ++t) {
+      const float4* r = A.rec + (int64_t)kRecQuads * t;
+      const float4 q0 = __ldg(r), q1 = __ldg(r + 1);
+      if (q0.w < 0.0f) continue;
+      const F3 ca = sub(c, xyz(q0));
+      float far = 0.0f, coords = 0.0f;
+      for (int v = 0; v < corners; ++v) {
+        const F3 x = xyz(__ldg(r + (v == 0 ? 0 : v + 1)));
+        far = fmaxf(far, norm(sub(x, c)));
+        coords += kSlack * abs1(x);
+      }
+      R = fmaxf(R, far * 1.0001f + coords + at_c);
+      // markers' normals need not have unit length
+      D = fmaxf(D, dot(ca, xyz(q1)) + q1.w + coords + (at_c + kSlack * abs1(ca)) * fmaxf(1.0f, abs1(xyz(q1))));
+    }
+  } else {
+    nlo = nhi = c;
+    if (any) R = D = inf;
+  }
+  float4* o = grp + (int64_t)kGrpQuads * g;
+  o[0] = make_float4(c.x, c.y, c.z, R);
+  o[1] = make_float4(nlo.x, nlo.y, nlo.z, D);
+  o[2] = make_float4(nhi.x, nhi.y, nhi.z, 0.0f);
 }
 
 // Distance and signed distance of node p to item t (hibm_mpm.py:5900-5920 /
@@ -540,84 +608,144 @@ __global__ void __launch_bounds__(256) k_ibs_search(SearchArgs A) {
 }
 
 // The far nodes k_ibs_search left open (hibm_mpm.py:5937-6010: internal when no
-// item at all sees the node outside, with the nearest of all items).  Every
-// item has to be looked at for every node, so what counts is the cost of a
-// look: a warp holds kFarNodes nodes, its lanes take the items of a tile that
-// the block has staged in shared memory (two quads an item), and an item is
-// evaluated in full only when its bound cannot tell that it is inside and
-// farther than the best so far.  One thread per node over all items took
-// 33.8 of the boundary rows' 34.2 ms on a 96 x 96 x 128 grid with 9,024
-// triangles: every evaluation formed the triangle's normal again, and the
-// internal nodes kept a few warps per SM busy with one serial chain each.  The
-// whole of the rows now takes 5.9 ms; the bound tests' issue slots are what is
-// left of it.
-constexpr int kFarNodes = 4, kFarWarps = 8, kFarTile = 256;
+// item at all sees the node outside, with the nearest of all items).  Items are
+// grouped by kGroup neighbours in index order (mesh order keeps them close to
+// each other), and a node asks a group's bounds (k_ibs_groups) before it asks
+// the items: can one of them see the node outside, can one be as near as the
+// best so far.  A warp holds kFarNodes nodes.
+//   1. Lanes over groups: the group whose centre is nearest.  Its items, one
+//      per lane for all the nodes at once, give the first best distance.
+//   2. Lanes over groups: the bounds.  Groups that pass are taken four at a
+//      time, an item per lane, which is evaluated in full only when its own
+//      bound cannot tell that it is inside and farther than the warp's best.
+// On a 96 x 96 x 128 grid with 9,024 triangles: one thread per node over all
+// items 33.8 ms; lanes over the items with their own bounds, each lane's best
+// its own, 4.86 ms; this 1.12 ms (the search and boundary rows around it 2.06
+// ms).  What is left is the group bounds' issue slots.
+constexpr int kFarNodes = 4, kFarWarps = 8;
+static_assert(kFarNodes * kGroup == 32, "one item per lane");
 
 __global__ void __launch_bounds__(kFarWarps * 32) k_ibs_far(SearchArgs A) {
-  __shared__ float4 tile[2][kFarTile];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
   const int64_t count = *A.far_count;
-  const int n = items(A);
-  constexpr int kPerBlock = kFarNodes * kFarWarps;
-  for (int64_t base = (int64_t)blockIdx.x * kPerBlock; base < count; base += (int64_t)gridDim.x * kPerBlock) {
+  const int n = items(A), ng = (n + kGroup - 1) / kGroup;
+  const int64_t stride = (int64_t)gridDim.x * kFarWarps * kFarNodes;
+  for (int64_t base = ((int64_t)blockIdx.x * kFarWarps + (threadIdx.x >> 5)) * kFarNodes; base < count; base += stride) {
     F3 p[kFarNodes];
-    float slack_p[kFarNodes];
-    Best best[kFarNodes];
-    unsigned open = 0;  // nodes of this warp that no item has seen outside
+    float near_d[kFarNodes];
+    int near_g[kFarNodes];
 #pragma unroll
     for (int q = 0; q < kFarNodes; ++q) {
-      const int64_t e = base + warp * kFarNodes + q;
+      const int64_t e = base + q;
       const int64_t c = A.far_nodes[e < count ? e : count - 1];
       p[q] = node_position(A, (int)(c / ((int64_t)A.ny * A.nz)), (int)((c / A.nz) % A.ny), (int)(c % A.nz));
-      slack_p[q] = kSlack * abs1(p[q]);
-      if (e < count) open |= 1u << q;
+      near_d[q] = __int_as_float(0x7f800000);
+      near_g[q] = 0;
     }
-    for (int t0 = 0; t0 < n; t0 += kFarTile) {
-      // also the barrier between the last tile's reads and this one's writes
-      if (!__syncthreads_or(open != 0)) break;
-      const int tn = min(kFarTile, n - t0);
-      for (int q = threadIdx.x; q < 2 * tn; q += blockDim.x)
-        tile[q & 1][q >> 1] = __ldg(A.rec + (int64_t)kRecQuads * (t0 + (q >> 1)) + (q & 1));
-      __syncthreads();
-      if (open == 0) continue;
-      for (int u = lane; u < tn; u += 32) {
-        const float4 q0 = tile[0][u], q1 = tile[1][u];
+    for (int g = lane; g < ng; g += 32) {
+      const F3 x = xyz(__ldg(A.grp + (int64_t)kGrpQuads * g));
 #pragma unroll
-        for (int q = 0; q < kFarNodes; ++q) {
-          const F3 off = sub(p[q], xyz(q0));
-          const float s = dot(off, xyz(q1)), lim = best[q].d + q0.w + slack_p[q];
-          const bool maybe_outside = s > A.tol - (q1.w + slack_p[q]);
-          const bool maybe_nearest = lim > 0.0f && dot(off, off) <= lim * lim;
-          if ((open >> q & 1u) && (maybe_outside || maybe_nearest)) {
-            float d, se;
-            item_eval(A, t0 + u, p[q], d, se);
-            if (se > A.tol)
-              open &= ~(1u << q);
-            else
-              best[q].offer(d, t0 + u);
-          }
+      for (int q = 0; q < kFarNodes; ++q) {
+        const F3 off = sub(p[q], x);
+        const float d2 = dot(off, off);
+        if (d2 < near_d[q]) {
+          near_d[q] = d2;
+          near_g[q] = g;
         }
       }
-      open = __reduce_and_sync(0xffffffffu, open);
     }
-    __syncthreads();  // the tile is staged again for the next nodes
+    // one item of the node's nearest group per lane
+    Best first;
+    bool outside = false;
+    {
+      const int q_own = lane / kGroup;
+      F3 p_own = p[0];
+      int g_own = 0;
 #pragma unroll
+      for (int q = 0; q < kFarNodes; ++q) {
+        // non-negative floats compare as their bit patterns; NaN lanes keep infinity
+        const unsigned m = __reduce_min_sync(kAll, __float_as_uint(near_d[q]));
+        const unsigned who = __ballot_sync(kAll, __float_as_uint(near_d[q]) == m);
+        const int g = __shfl_sync(kAll, near_g[q], __ffs(who) - 1);
+        if (q == q_own) {
+          p_own = p[q];
+          g_own = g;
+        }
+      }
+      const int t = g_own * kGroup + (lane & (kGroup - 1));
+      if (t < n && __ldg(A.rec + (int64_t)kRecQuads * t).w >= 0.0f) {
+        float d, s;
+        item_eval(A, t, p_own, d, s);
+        outside = s > A.tol;
+        first.offer(d, t);
+      }
+    }
+    const unsigned seen = __ballot_sync(kAll, outside);
     for (int q = 0; q < kFarNodes; ++q) {
-      // the lanes' lexicographic minima of (distance, index)
-      Best b = best[q];
+      if (base + q >= count || (seen >> (q * kGroup) & ((1u << kGroup) - 1u))) continue;
+      const F3 pq = q == 0 ? p[0] : q == 1 ? p[1] : q == 2 ? p[2] : p[3];
+      const float slack_p = kSlack * abs1(pq);
+      Best best;
+      if (lane / kGroup == q) best = first;
+      float bound = __uint_as_float(__reduce_min_sync(kAll, __float_as_uint(best.d)));
+      bool open = true;  // no item has seen the node outside
+      for (int g0 = 0; open && g0 < ng; g0 += 32) {
+        bool ask = false;
+        if (g0 + lane < ng) {
+          const float4* r = A.grp + (int64_t)kGrpQuads * (g0 + lane);
+          const float4 q0 = __ldg(r), q1 = __ldg(r + 1), q2 = __ldg(r + 2);
+          const F3 off = sub(pq, xyz(q0));
+          const float lim = bound + q0.w + slack_p;
+          const float up = fmaxf(off.x * q1.x, off.x * q2.x) + fmaxf(off.y * q1.y, off.y * q2.y) +
+                           fmaxf(off.z * q1.z, off.z * q2.z);
+          ask = (lim > 0.0f && dot(off, off) <= lim * lim) || up > A.tol - (q1.w + 2.0f * slack_p);
+        }
+        unsigned todo = __ballot_sync(kAll, ask);
+        while (todo != 0) {
+          // lanes kGroup * w .. take the w-th group asked; then those are done
+          unsigned own = todo;
+#pragma unroll
+          for (int w = 0; w < kFarNodes; ++w) {
+            if (w < lane / kGroup) own &= own - 1;
+            todo &= todo - 1;
+          }
+          bool out = false;
+          const int t = (g0 + __ffs(own) - 1) * kGroup + (lane & (kGroup - 1));
+          if (own != 0 && t < n) {
+            const float4 q0 = __ldg(A.rec + (int64_t)kRecQuads * t), q1 = __ldg(A.rec + (int64_t)kRecQuads * t + 1);
+            const F3 off = sub(pq, xyz(q0));
+            const float lim = bound + q0.w + slack_p;
+            if (dot(off, xyz(q1)) > A.tol - (q1.w + slack_p) || (lim > 0.0f && dot(off, off) <= lim * lim)) {
+              float d, s;
+              item_eval(A, t, pq, d, s);
+              out = s > A.tol;
+              if (!out) best.offer(d, t);
+            }
+          }
+          if (__any_sync(kAll, out)) {
+            open = false;
+            break;
+          }
+          bound = fminf(bound, __uint_as_float(__reduce_min_sync(kAll, __float_as_uint(best.d))));
+        }
+      }
+      if (!open) continue;
+      // the lanes' lexicographic minimum of (distance, index)
+      Best b = best;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
-        const float d = __shfl_xor_sync(0xffffffffu, b.d, o);
-        const int t = __shfl_xor_sync(0xffffffffu, b.t, o);
+        const float d = __shfl_xor_sync(kAll, b.d, o);
+        const int t = __shfl_xor_sync(kAll, b.t, o);
         if (t >= 0) b.offer(d, t);
       }
-      if (!(open >> q & 1u) || b.t < 0 || lane != 0) continue;
+      if (b.t < 0 || lane != 0) continue;
       int marker, ix[3];
       float w[3], d, sd;
       F3 boundary, normal;
-      item_detail(A, b.t, p[q], marker, boundary, normal, ix, w);
-      item_eval(A, b.t, p[q], d, sd);
-      const int64_t c = A.far_nodes[base + warp * kFarNodes + q];
+      item_detail(A, b.t, pq, marker, boundary, normal, ix, w);
+      item_eval(A, b.t, pq, d, sd);
+      const int64_t c = A.far_nodes[base + q];
       A.kind[c] = kNodeInternal;
       A.nearest[c] = marker;
       A.sd[c] = sd;
@@ -1113,6 +1241,7 @@ int efsi_ib_search_plan_destroy(efsi_ib_search_plan* P) {
   cudaFree(P->entries);
   cudaFree(P->claim);
   cudaFree(P->rec);
+  cudaFree(P->grp);
   cudaFree(P->far_nodes);
   cudaFree(P->far_count);
   cudaFree(P->total);
@@ -1218,6 +1347,12 @@ int efsi_ib_node_search(efsi_ib_search_plan* P, const efsi_ib_search_params* prm
   }
   if (nitems > 0) {
     EFSI_COUNTED k_ibs_records<<<(unsigned)((nitems + 255) / 256), 256, 0, s>>>(A, P->rec);
+    if (A.classify_far) {
+      const int ng = (nitems + kGroup - 1) / kGroup;
+      EFSI_TRY(grow(P->grp, P->grp_cap, (int64_t)kGrpQuads * ng));
+      A.grp = P->grp;
+      EFSI_COUNTED k_ibs_groups<<<(unsigned)((ng + 63) / 64), 64, 0, s>>>(A, P->grp);
+    }
     const int64_t tiles = (nbins + kScanTile - 1) / kScanTile;
     if (nbins > P->bin_cap) {
       cudaFree(P->count);

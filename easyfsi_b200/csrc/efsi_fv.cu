@@ -770,8 +770,8 @@ struct TailDesc {
   LevelDev L[kTailMaxLevels];
   int foff[kTailMaxLevels];  // float offset of level l's block (pA, pB, rhs) in shared memory
   int moff[kTailMaxLevels];  // byte offset of level l's mask copy
-  int coff[kTailMaxLevels];  // byte offset of level l's row table: 6 face coefficients + denominator (f64, SoA)
-  int noff[kTailMaxLevels];  // byte offset of level l's neighbour table: 6 cell indices (int, SoA)
+  int coff[kTailMaxLevels];  // byte offset of level l's row table: 6 face coefficients, denominator, 1 / denominator (f64, SoA)
+  int noff[kTailMaxLevels];  // byte offset of level l's neighbour table: 6 cell indices (16 bits, SoA)
   const float* rhs_in;       // rhs of level lt (written by the restriction from lt - 1)
   float* p_out;              // final iterate of level lt
 };
@@ -793,7 +793,8 @@ __device__ __forceinline__ void tail_ijk(const LevelDev& L, int t, int& i, int& 
 struct TailTables {
   const double* a;  // [6][n]
   const double* den;  // [n]
-  const int* nb;  // [6][n]
+  const double* rden;  // [n]: 1 / den, 0 where the row's result is 0
+  const uint16_t* nb;  // [6][n]
   int n;
 };
 
@@ -803,7 +804,8 @@ __device__ __forceinline__ TailTables tail_tables(const TailDesc& T, int l, unsi
   tb.n = L.nx * L.ny * L.nz;
   tb.a = reinterpret_cast<const double*>(smem + T.coff[l]);
   tb.den = tb.a + 6 * tb.n;
-  tb.nb = reinterpret_cast<const int*>(smem + T.noff[l]);
+  tb.rden = tb.a + 7 * tb.n;
+  tb.nb = reinterpret_cast<const uint16_t*>(smem + T.noff[l]);
   return tb;
 }
 
@@ -812,7 +814,8 @@ __device__ void tail_build_tables(const TailDesc& T, int l, unsigned char* smem,
   const int n = L.nx * L.ny * L.nz;
   double* a = reinterpret_cast<double*>(smem + T.coff[l]);
   double* den = a + 6 * n;
-  int* nb = reinterpret_cast<int*>(smem + T.noff[l]);
+  double* rden = a + 7 * n;
+  uint16_t* nb = reinterpret_cast<uint16_t*>(smem + T.noff[l]);
   const int sx = L.ny * L.nz, sy = L.nz;
   for (int t = threadIdx.x; t < n; t += blockDim.x) {
     int i, j, k;
@@ -838,13 +841,24 @@ __device__ void tail_build_tables(const TailDesc& T, int l, unsigned char* smem,
     for (int f = 0; f < 6; ++f) {
       const double af = (m & bit[f]) ? kf[f] : 0.0;
       a[f * n + t] = af;
-      nb[f * n + t] = c[f];
+      nb[f * n + t] = (uint16_t)c[f];
       d = d + af;
     }
     if (T.outlet && k == 0) d += L.oz;
     d += iface_at<float>(L, t);
     den[t] = d;
+    rden[t] = !(m & M_SOLID) && d > 0.0 ? 1.0 / d : 0.0;
   }
+}
+
+// x / w with r = 1 / w rounded to nearest: the product corrected by its exact
+// remainder rounds as the quotient does while nothing underflows (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990); a remainder that is not finite leaves the product.
+__device__ __forceinline__ double tail_div(double x, double w, double r) {
+  const double q = x * r;
+  const double e = fma(-q, w, x);
+  return fabs(e) <= 1.7e308 ? fma(e, r, q) : q;
 }
 
 // Neighbour sum of row t from the tables (same order and fused multiply-adds
@@ -857,23 +871,75 @@ __device__ __forceinline__ double tail_ns(const TailTables& tb, const float* p, 
 }
 
 // One Jacobi sweep of level l: src -> dst (src null: zero initial guess).
-__device__ void tail_sweep(const TailTables& tb, const float* src, float* dst, const float* rhs, const uint8_t* mask,
-                           double omega) {
+__device__ void tail_sweep(const TailTables& tb, const float* src, float* dst, const float* rhs, double omega) {
   for (int t = threadIdx.x; t < tb.n; t += blockDim.x) {
-    const unsigned m = mask[t];
+    const double rd = tb.rden[t];
     float res = 0.0f;
-    if (!(m & M_SOLID)) {
-      const double den = tb.den[t];
-      if (den > 0.0) {
-        const double ns = src != nullptr ? tail_ns(tb, src, t) : 0.0;
-        const double jv = (ns - (double)rhs[t]) / den;
-        const double pcur = src != nullptr ? (double)src[t] : 0.0;
-        res = (float)(pcur + omega * (jv - pcur));
-      }
+    if (rd != 0.0) {
+      const double ns = src != nullptr ? tail_ns(tb, src, t) : 0.0;
+      const double jv = tail_div(ns - (double)rhs[t], tb.den[t], rd);
+      const double pcur = src != nullptr ? (double)src[t] : 0.0;
+      res = (float)(pcur + omega * (jv - pcur));
     }
     dst[t] = res;
   }
   __syncthreads();
+}
+
+// `sweeps` Jacobi sweeps of a level with at most one cell per thread,
+// alternating between the two buffers; returns the one that holds the result
+// (c: the one that holds the start, -1 for zero).  A row's coefficients stay
+// in registers, and only the warps that hold cells meet at the barrier between
+// sweeps: a sweep of a handful of cells is the latency of that barrier, of six
+// shared loads and of a dozen dependent f64 operations.
+__device__ int tail_sweeps_small(const TailTables& tb, float* const buf[2], int c, int sweeps, const float* rhs,
+                                 double omega) {
+  const int t = threadIdx.x, active = (tb.n + 31) & ~31;
+  if (t < active) {
+    const int u = min(t, tb.n - 1);
+    double a[6];
+    int nb[6];
+#pragma unroll
+    for (int f = 0; f < 6; ++f) {
+      a[f] = tb.a[f * tb.n + u];
+      nb[f] = tb.nb[f * tb.n + u];
+    }
+    const double den = tb.den[u], rd = tb.rden[u], b = (double)rhs[u];
+    float p = c < 0 ? 0.0f : buf[c][u];
+    for (int it = 0; it < sweeps; ++it) {
+      double ns = 0.0;
+      if (c >= 0) {
+        const float* src = buf[c];
+        ns = fma(a[0], (double)src[nb[0]], 0.0);
+#pragma unroll
+        for (int f = 1; f < 6; ++f) ns = fma(a[f], (double)src[nb[f]], ns);
+      }
+      const double pcur = (double)p;
+      const double jv = tail_div(ns - b, den, rd);
+      p = rd != 0.0 ? (float)(pcur + omega * (jv - pcur)) : 0.0f;
+      c = c < 0 ? 0 : 1 - c;
+      if (t < tb.n) buf[c][t] = p;
+      if (active == 32)
+        __syncwarp();
+      else
+        asm volatile("bar.sync 1, %0;" ::"r"(active) : "memory");
+    }
+  } else if (sweeps > 0) {
+    c = c < 0 ? (sweeps - 1) & 1 : (c + sweeps) & 1;
+  }
+  __syncthreads();
+  return c;
+}
+
+__device__ int tail_sweeps(const TailTables& tb, float* const buf[2], int c, int sweeps, const float* rhs,
+                           double omega) {
+  if (tb.n <= (int)blockDim.x) return tail_sweeps_small(tb, buf, c, sweeps, rhs, omega);
+  for (int it = 0; it < sweeps; ++it) {
+    const int d = c < 0 ? 0 : 1 - c;
+    tail_sweep(tb, c < 0 ? nullptr : buf[c], buf[d], rhs, omega);
+    c = d;
+  }
+  return c;
 }
 
 // p += s * p_coarse on the fluid cells of level l (fluid.py:5391-5406).
@@ -892,44 +958,53 @@ __device__ void tail_prolong(const TailDesc& T, int l, float* p, const uint8_t* 
 }
 
 // Residual of level l formed from the tables and volume-weighted into the
-// rhs of l+1 (fluid.py:5262-5388).
+// rhs of l+1 (fluid.py:5262-5388).  Eight lanes form a coarse cell's eight
+// residuals; its sum is folded over them in the reference's order.
 __device__ void tail_restrict(const TailDesc& T, int l, const TailTables& tb, const float* p, const float* rhs,
                               const uint8_t* mask, float* crhs) {
   const LevelDev& F = T.L[l];
   const LevelDev& C = T.L[l + 1];
-  const int nc = C.nx * C.ny * C.nz;
-  for (int t = threadIdx.x; t < nc; t += blockDim.x) {
-    int i, j, k;
-    tail_ijk(C, t, i, j, k);
-    float wres = 0.0f, free_vol = 0.0f;
-    int ocount = 0;
-    for (int oi = 0; oi < 2; ++oi)
-      for (int oj = 0; oj < 2; ++oj)
-        for (int ok = 0; ok < 2; ++ok) {
-          const int fi = 2 * i + oi, fj = 2 * j + oj, fk = 2 * k + ok;
-          if (fi < F.nx && fj < F.ny && fk < F.nz) {
-            const int f = (fi * F.ny + fj) * F.nz + fk;
-            if (mask[f] & M_SOLID) {
-              ocount += 1;
-            } else {
-              const float vol = __fmul_rn(__fmul_rn(__ldg(F.wx + fi), __ldg(F.wy + fj)), __ldg(F.wz + fk));
-              const double ns = tail_ns(tb, p, f);
-              const float r = (float)((double)rhs[f] - (ns - tb.den[f] * (double)p[f]));
-              wres = __fadd_rn(wres, __fmul_rn(r, vol));
-              free_vol = __fadd_rn(free_vol, vol);
-            }
-          }
+  const int n8 = 8 * C.nx * C.ny * C.nz, lane = threadIdx.x & 31;
+  for (int base = threadIdx.x - lane; base < n8; base += blockDim.x) {
+    const int t = (base + lane) >> 3, ch = lane & 7;
+    bool solid = false;
+    float rv = 0.0f, vol = 0.0f;
+    if (base + lane < n8) {
+      int i, j, k;
+      tail_ijk(C, t, i, j, k);
+      const int fi = 2 * i + (ch >> 2), fj = 2 * j + ((ch >> 1) & 1), fk = 2 * k + (ch & 1);
+      if (fi < F.nx && fj < F.ny && fk < F.nz) {
+        const int f = (fi * F.ny + fj) * F.nz + fk;
+        solid = (mask[f] & M_SOLID) != 0;
+        if (!solid) {
+          vol = __fmul_rn(__fmul_rn(__ldg(F.wx + fi), __ldg(F.wy + fj)), __ldg(F.wz + fk));
+          const double ns = tail_ns(tb, p, f);
+          rv = __fmul_rn((float)((double)rhs[f] - (ns - tb.den[f] * (double)p[f])), vol);
         }
-    crhs[t] = ocount > 0 ? 0.0f : __fdiv_rn(wres, fmaxf(free_vol, 1.0e-30f));
+      }
+    }
+    float wres = 0.0f, free_vol = 0.0f;
+#pragma unroll
+    for (int o = 0; o < 8; ++o) {
+      wres = __fadd_rn(wres, __shfl_sync(0xffffffffu, rv, (lane & ~7) + o));
+      free_vol = __fadd_rn(free_vol, __shfl_sync(0xffffffffu, vol, (lane & ~7) + o));
+    }
+    const bool any_solid = (__ballot_sync(0xffffffffu, solid) >> (lane & ~7) & 0xffu) != 0;
+    if (ch == 0 && base + lane < n8) crhs[t] = any_solid ? 0.0f : __fdiv_rn(wres, fmaxf(free_vol, 1.0e-30f));
   }
   __syncthreads();
 }
 
-// The whole tail V-cycle by one CTA (all threads of the block take part).
+// Row tables and masks of every tail level.  They depend on the level's
+// structure alone, which no kernel of a V-cycle changes.
+__device__ void tail_prologue(const TailDesc& T, unsigned char* tail_smem) {
+  for (int l = T.lt; l < T.nl; ++l) tail_build_tables(T, l, tail_smem, tail_smem + T.moff[l]);
+}
+
+// The whole tail V-cycle by one CTA (all threads of the block take part),
+// after tail_prologue.
 __device__ void tail_body(const TailDesc& T, unsigned char* tail_smem) {
   float* fpool = reinterpret_cast<float*>(tail_smem);
-  // row tables and masks of every tail level, the rhs of level lt
-  for (int l = T.lt; l < T.nl; ++l) tail_build_tables(T, l, tail_smem, tail_smem + T.moff[l]);
   {
     const LevelDev& L = T.L[T.lt];
     const int n = L.nx * L.ny * L.nz;
@@ -948,12 +1023,7 @@ __device__ void tail_body(const TailDesc& T, unsigned char* tail_smem) {
     const TailTables tb = tail_tables(T, l, tail_smem);
     const bool coarsest = (l == T.nl - 1);
     const int sweeps = coarsest ? T.coarse : T.pre;
-    int c = -1;
-    for (int it = 0; it < sweeps; ++it) {
-      const int d = (it & 1);
-      tail_sweep(tb, c < 0 ? nullptr : buf[c], buf[d], rhs, ms, T.omega);
-      c = d;
-    }
+    const int c = tail_sweeps(tb, buf, -1, sweeps, rhs, T.omega);
     cur[l] = c;
     if (!coarsest) {
       const LevelDev& C = T.L[l + 1];
@@ -971,14 +1041,8 @@ __device__ void tail_body(const TailDesc& T, unsigned char* tail_smem) {
     const TailTables tb = tail_tables(T, l, tail_smem);
     const LevelDev& C = T.L[l + 1];
     const float* pc = fpool + T.foff[l + 1] + cur[l + 1] * (C.nx * C.ny * C.nz);
-    int c = cur[l];
-    tail_prolong(T, l, buf[c], ms, pc);
-    for (int it = 0; it < T.post; ++it) {
-      const int d = 1 - c;
-      tail_sweep(tb, buf[c], buf[d], rhs, ms, T.omega);
-      c = d;
-    }
-    cur[l] = c;
+    tail_prolong(T, l, buf[cur[l]], ms, pc);
+    cur[l] = tail_sweeps(tb, buf, cur[l], T.post, rhs, T.omega);
   }
   {
     const LevelDev& L = T.L[T.lt];
@@ -989,8 +1053,12 @@ __device__ void tail_body(const TailDesc& T, unsigned char* tail_smem) {
 }
 
 __global__ void __launch_bounds__(kTailThreads) k_mg_tail(TailDesc T) {
-  pdl_wait();
   extern __shared__ __align__(16) unsigned char tail_smem[];
+  // While the kernel before (the restriction into level lt) still runs: it
+  // started after everything before it was complete, the tables' inputs
+  // included, and writes none of them.
+  tail_prologue(T, tail_smem);
+  pdl_wait();
   tail_body(T, tail_smem);
 }
 
@@ -1208,7 +1276,10 @@ __global__ void __launch_bounds__(kTailThreads) k_mg_coarse(const __grid_constan
     }
   }
   if (!coarse_barrier(D)) return;
-  if (blockIdx.x == 0) tail_body(T, tail_smem);
+  if (blockIdx.x == 0) {
+    tail_prologue(T, tail_smem);
+    tail_body(T, tail_smem);
+  }
   if (!coarse_barrier(D)) return;
   // up
   const float* fin = T.p_out;  // final iterate of level l + 1
@@ -2078,7 +2149,7 @@ static void preload_kernels() {
 
 namespace efsi {
 // Picks the first coarse level from which every level fits the tail kernel's
-// shared memory (13 bytes per cell) and has at most EFSI_TAIL_MAX_CELLS cells
+// shared memory (89 bytes per cell) and has at most EFSI_TAIL_MAX_CELLS cells
 // (default 4096; 0 disables the tail).
 static void configure_tail(efsi_fv_plan* P) {
   P->tail_level = P->n_levels;
@@ -2089,26 +2160,28 @@ static void configure_tail(efsi_fv_plan* P) {
   cudaGetDevice(&dev);
   int smem_optin = 0;
   cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  max_cells = std::min(max_cells, 65535);  // 16-bit neighbour indices
   for (int lt = 1; lt < P->n_levels; ++lt) {
     if (P->lv[lt].n > max_cells) continue;
-    // layout: row tables (7 f64 per cell), iterates + rhs (3 f32 per cell),
-    // neighbour tables (6 int per cell), masks (1 byte per cell, 16-aligned)
+    // layout: row tables (8 f64 per cell), iterates + rhs (3 f32 per cell),
+    // neighbour tables (6 16-bit indices per cell), masks (1 byte per cell,
+    // 16-aligned)
     size_t cells = 0, bytes_mask = 0;
     for (int l = lt; l < P->n_levels; ++l) {
       cells += (size_t)P->lv[l].n;
       bytes_mask += ((size_t)P->lv[l].n + 15) / 16 * 16;
     }
-    const size_t total = cells * (7 * sizeof(double) + 3 * sizeof(float) + 6 * sizeof(int)) + bytes_mask;
+    const size_t total = cells * (8 * sizeof(double) + 3 * sizeof(float) + 6 * sizeof(uint16_t)) + 16 + bytes_mask;
     if ((int64_t)total > (int64_t)smem_optin) continue;
-    size_t co = 0, fo = cells * 7 * sizeof(double), no = fo + cells * 3 * sizeof(float), mo = no + cells * 6 * sizeof(int);
+    size_t co = 0, fo = cells * 8 * sizeof(double), no = fo + cells * 3 * sizeof(float), mo = (no + cells * 6 * sizeof(uint16_t) + 15) / 16 * 16;
     for (int l = lt; l < P->n_levels; ++l) {
       const size_t n = (size_t)P->lv[l].n;
       P->tail_coff[l] = (int)co;
-      co += n * 7 * sizeof(double);
+      co += n * 8 * sizeof(double);
       P->tail_foff[l] = (int)(fo / sizeof(float));
       fo += n * 3 * sizeof(float);
       P->tail_noff[l] = (int)no;
-      no += n * 6 * sizeof(int);
+      no += n * 6 * sizeof(uint16_t);
       P->tail_moff[l] = (int)mo;
       mo += (n + 15) / 16 * 16;
     }

@@ -382,134 +382,175 @@ __device__ __forceinline__ double warp_allsum(double v) {
   return v;
 }
 
+// The markers of one block (a warp each, kMarkerWarps at a time) report
+// together: every warp's lane 0 keeps its sums and maxima, and the block adds
+// them once.  With an atomic per marker and value, 65,000 of them on one cache
+// line took most of the exchange of 8,192 markers: the scatter 87 us, the
+// feedback 59; now @SC@ and @FB@.
+constexpr int kMarkerWarps = 8;
+
+// The larger of two non-negative values by their bits, as atomic_max_nonneg_d
+// takes them: a NaN wins.
+__device__ __forceinline__ double max_nonneg(double a, double b) {
+  return (unsigned long long)__double_as_longlong(a) < (unsigned long long)__double_as_longlong(b) ? b : a;
+}
+
+// Adds (max_mask: keeps the larger of) the block's values; every thread takes part.
+template <int N>
+__device__ __forceinline__ void block_report(const double (&v)[N], unsigned max_mask, double* rep) {
+  __shared__ double part[kMarkerWarps][N];
+  if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+    for (int q = 0; q < N; ++q) part[threadIdx.x >> 5][q] = v[q];
+  }
+  __syncthreads();
+  if (threadIdx.x < N) {
+    const int q = (int)threadIdx.x;
+    const bool mx = (max_mask >> q) & 1u;
+    double t = part[0][q];
+    for (int w = 1; w < kMarkerWarps; ++w) t = mx ? max_nonneg(t, part[w][q]) : t + part[w][q];
+    if (mx)
+      atomic_max_nonneg_d(rep + q, t);
+    else if (t != 0.0)  // (a sum that is NaN is added)
+      atomicAdd(rep + q, t);
+  }
+}
+
 // hibm_mpm.py:4899-4959 _scatter_marker_forces_to_mpm_particles_kernel: one
 // warp per marker; the tent-weight sum over the marker's neighbourhood is a
 // warp reduction, then the lanes spread F * w / wsum to the particles.
-__global__ void k_scatter(BinView B, int M, const float* xg, const double* Fg, const float* xp, float* fext,
-                          double* rep) {
-  const int m = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = (int)(threadIdx.x & 31);
-  if (m >= M) return;  // uniform over the warp
-  const float xm[3] = {__ldg(xg + 3 * m), __ldg(xg + 3 * m + 1), __ldg(xg + 3 * m + 2)};
-  const double Fm[3] = {__ldg(Fg + 3 * m), __ldg(Fg + 3 * m + 1), __ldg(Fg + 3 * m + 2)};
-  const bool valid = finite3(xm) && isfinite(Fm[0]) && isfinite(Fm[1]) && isfinite(Fm[2]);
-  const float R = B.R;
-  float wl = 0.0f;
-  if (valid) for_near(B, xm, lane, [&](int p) { wl += tent(xm, xp + 3 * p, R); });
-  const float wsum = warp_allsum(wl);
-  if (valid && wsum > 1.0e-12f) {
-    double e0 = 0, e1 = 0, e2 = 0, contrib = 0;
-    for_near(B, xm, lane, [&](int p) {
-      float w = tent(xm, xp + 3 * p, R);
-      if (w > 0.0f) {
-        const double ratio = (double)(w / wsum);
-        float f0 = (float)(Fm[0] * ratio), f1 = (float)(Fm[1] * ratio), f2 = (float)(Fm[2] * ratio);
-        atomicAdd(fext + 3 * p, f0);
-        atomicAdd(fext + 3 * p + 1, f1);
-        atomicAdd(fext + 3 * p + 2, f2);
-        e0 += f0;
-        e1 += f1;
-        e2 += f2;
-        contrib += 1.0;
-      }
-    });
-    e0 = warp_allsum(e0);
-    e1 = warp_allsum(e1);
-    e2 = warp_allsum(e2);
-    contrib = warp_allsum(contrib);
-    if (lane == 0) {
-      atomicAdd(rep + 0, 1.0);
-      atomicAdd(rep + 3, Fm[0]);
-      atomicAdd(rep + 4, Fm[1]);
-      atomicAdd(rep + 5, Fm[2]);
-      atomicAdd(rep + 2, contrib);
-      atomicAdd(rep + 6, e0);
-      atomicAdd(rep + 7, e1);
-      atomicAdd(rep + 8, e2);
+__global__ void __launch_bounds__(32 * kMarkerWarps) k_scatter(BinView B, int M, const float* xg, const double* Fg,
+                                                               const float* xp, float* fext, double* rep) {
+  const int lane = (int)(threadIdx.x & 31);
+  double tot[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  for (int m = (int)(blockIdx.x * kMarkerWarps + (threadIdx.x >> 5)); m < M; m += (int)gridDim.x * kMarkerWarps) {
+    const float xm[3] = {__ldg(xg + 3 * m), __ldg(xg + 3 * m + 1), __ldg(xg + 3 * m + 2)};
+    const double Fm[3] = {__ldg(Fg + 3 * m), __ldg(Fg + 3 * m + 1), __ldg(Fg + 3 * m + 2)};
+    const bool valid = finite3(xm) && isfinite(Fm[0]) && isfinite(Fm[1]) && isfinite(Fm[2]);
+    const float R = B.R;
+    float wl = 0.0f;
+    if (valid) for_near(B, xm, lane, [&](int p) { wl += tent(xm, xp + 3 * p, R); });
+    const float wsum = warp_allsum(wl);
+    if (valid && wsum > 1.0e-12f) {
+      double e0 = 0, e1 = 0, e2 = 0, contrib = 0;
+      for_near(B, xm, lane, [&](int p) {
+        float w = tent(xm, xp + 3 * p, R);
+        if (w > 0.0f) {
+          const double ratio = (double)(w / wsum);
+          float f0 = (float)(Fm[0] * ratio), f1 = (float)(Fm[1] * ratio), f2 = (float)(Fm[2] * ratio);
+          atomicAdd(fext + 3 * p, f0);
+          atomicAdd(fext + 3 * p + 1, f1);
+          atomicAdd(fext + 3 * p + 2, f2);
+          e0 += f0;
+          e1 += f1;
+          e2 += f2;
+          contrib += 1.0;
+        }
+      });
+      tot[0] += 1.0;
+      tot[2] += warp_allsum(contrib);
+      tot[3] += Fm[0];
+      tot[4] += Fm[1];
+      tot[5] += Fm[2];
+      tot[6] += warp_allsum(e0);
+      tot[7] += warp_allsum(e1);
+      tot[8] += warp_allsum(e2);
+    } else {
+      tot[1] += 1.0;
     }
-  } else if (lane == 0) {
-    atomicAdd(rep + 1, 1.0);
   }
+  block_report(tot, 0u, rep);
 }
 
 // hibm_mpm.py:5097-5180 / 5012-5053 surface feedback: one warp per marker,
 // tent-weighted sums of particle velocity (and normal / area) as warp
 // reductions.
-__global__ void k_feedback(BinView B, int M, float* xg, float* vg, float* ng, float* Ag, const float* xp,
-                           const float* vp, const float* np_, const float* ap, float dt, double* rep) {
-  const int m = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = (int)(threadIdx.x & 31);
-  if (m >= M) return;  // uniform over the warp
+__global__ void __launch_bounds__(32 * kMarkerWarps) k_feedback(BinView B, int M, float* xg, float* vg, float* ng,
+                                                                float* Ag, const float* xp, const float* vp,
+                                                                const float* np_, const float* ap, float dt,
+                                                                double* rep) {
+  const int lane = (int)(threadIdx.x & 31);
   const bool geometry = np_ != nullptr && ap != nullptr;
-  const float xo[3] = {xg[3 * m], xg[3 * m + 1], xg[3 * m + 2]};
-  const float no[3] = {ng[3 * m], ng[3 * m + 1], ng[3 * m + 2]};
-  const float ao = Ag[m];
-  float vs[3] = {0, 0, 0}, ns[3] = {0, 0, 0}, as = 0.0f, ws = 0.0f, gs = 0.0f;
-  const float R = B.R;
-  for_near(B, xo, lane, [&](int p) {
-    float w = tent(xo, xp + 3 * p, R);
-    if (w > 0.0f) {
-      vs[0] += w * __ldg(vp + 3 * p);
-      vs[1] += w * __ldg(vp + 3 * p + 1);
-      vs[2] += w * __ldg(vp + 3 * p + 2);
-      ws += w;
-      if (geometry) {
-        const float* pn = np_ + 3 * p;
-        if (sqrtf(pn[0] * pn[0] + pn[1] * pn[1] + pn[2] * pn[2]) > 1.0e-12f && ap[p] > 0.0f) {
-          ns[0] += w * pn[0];
-          ns[1] += w * pn[1];
-          ns[2] += w * pn[2];
-          as += w * ap[p];
-          gs += w;
+  double tot[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // four counts, four maxima
+  for (int m = (int)(blockIdx.x * kMarkerWarps + (threadIdx.x >> 5)); m < M; m += (int)gridDim.x * kMarkerWarps) {
+    const float xo[3] = {xg[3 * m], xg[3 * m + 1], xg[3 * m + 2]};
+    const float no[3] = {ng[3 * m], ng[3 * m + 1], ng[3 * m + 2]};
+    const float ao = Ag[m];
+    float vs[3] = {0, 0, 0}, ns[3] = {0, 0, 0}, as = 0.0f, ws = 0.0f, gs = 0.0f;
+    const float R = B.R;
+    for_near(B, xo, lane, [&](int p) {
+      float w = tent(xo, xp + 3 * p, R);
+      if (w > 0.0f) {
+        vs[0] += w * __ldg(vp + 3 * p);
+        vs[1] += w * __ldg(vp + 3 * p + 1);
+        vs[2] += w * __ldg(vp + 3 * p + 2);
+        ws += w;
+        if (geometry) {
+          const float* pn = np_ + 3 * p;
+          if (sqrtf(pn[0] * pn[0] + pn[1] * pn[1] + pn[2] * pn[2]) > 1.0e-12f && ap[p] > 0.0f) {
+            ns[0] += w * pn[0];
+            ns[1] += w * pn[1];
+            ns[2] += w * pn[2];
+            as += w * ap[p];
+            gs += w;
+          }
         }
       }
-    }
-  });
+    });
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    vs[a] = warp_allsum(vs[a]);
-    ns[a] = warp_allsum(ns[a]);
-  }
-  as = warp_allsum(as);
-  ws = warp_allsum(ws);
-  gs = warp_allsum(gs);
-  if (lane != 0) return;
-  if (ws > 1.0e-12f) {
-    float nv[3], nx[3];
     for (int a = 0; a < 3; ++a) {
-      nv[a] = vs[a] / ws;
-      nx[a] = xo[a] + dt * nv[a];
-      xg[3 * m + a] = nx[a];
-      vg[3 * m + a] = nv[a];
+      vs[a] = warp_allsum(vs[a]);
+      ns[a] = warp_allsum(ns[a]);
     }
-    atomicAdd(rep + 0, 1.0);
-    double dd = 0, sp = 0;
-    for (int a = 0; a < 3; ++a) {
-      dd += (double)(nx[a] - xo[a]) * (nx[a] - xo[a]);
-      sp += (double)nv[a] * nv[a];
-    }
-    atomic_max_nonneg_d(rep + 4, sqrt(dd));
-    atomic_max_nonneg_d(rep + 5, sqrt(sp));
-    if (geometry) {
-      float nn = sqrtf(ns[0] * ns[0] + ns[1] * ns[1] + ns[2] * ns[2]);
-      if (gs > 1.0e-12f && nn > 1.0e-12f) {
-        double dn = 0;
-        for (int a = 0; a < 3; ++a) {
-          float v = ns[a] / nn;
-          ng[3 * m + a] = v;
-          dn += (double)(v - no[a]) * (v - no[a]);
-        }
-        float na = as / gs;
-        Ag[m] = na;
-        atomicAdd(rep + 2, 1.0);
-        atomic_max_nonneg_d(rep + 6, sqrt(dn));
-        atomic_max_nonneg_d(rep + 7, (double)fabsf(na - ao));
-      } else {
-        atomicAdd(rep + 3, 1.0);
+    as = warp_allsum(as);
+    ws = warp_allsum(ws);
+    gs = warp_allsum(gs);
+    if (lane != 0) continue;
+    if (ws > 1.0e-12f) {
+      float nv[3], nx[3];
+      for (int a = 0; a < 3; ++a) {
+        nv[a] = vs[a] / ws;
+        nx[a] = xo[a] + dt * nv[a];
+        xg[3 * m + a] = nx[a];
+        vg[3 * m + a] = nv[a];
       }
+      tot[0] += 1.0;
+      double dd = 0, sp = 0;
+      for (int a = 0; a < 3; ++a) {
+        dd += (double)(nx[a] - xo[a]) * (nx[a] - xo[a]);
+        sp += (double)nv[a] * nv[a];
+      }
+      tot[4] = max_nonneg(tot[4], sqrt(dd));
+      tot[5] = max_nonneg(tot[5], sqrt(sp));
+      if (geometry) {
+        float nn = sqrtf(ns[0] * ns[0] + ns[1] * ns[1] + ns[2] * ns[2]);
+        if (gs > 1.0e-12f && nn > 1.0e-12f) {
+          double dn = 0;
+          for (int a = 0; a < 3; ++a) {
+            float v = ns[a] / nn;
+            ng[3 * m + a] = v;
+            dn += (double)(v - no[a]) * (v - no[a]);
+          }
+          float na = as / gs;
+          Ag[m] = na;
+          tot[2] += 1.0;
+          tot[6] = max_nonneg(tot[6], sqrt(dn));
+          tot[7] = max_nonneg(tot[7], (double)fabsf(na - ao));
+        } else {
+          tot[3] += 1.0;
+        }
+      }
+    } else {
+      tot[1] += 1.0;
+      if (geometry) tot[3] += 1.0;
     }
-  } else {
-    atomicAdd(rep + 1, 1.0);
-    if (geometry) atomicAdd(rep + 3, 1.0);
   }
+  block_report(tot, 0xF0u, rep);
+}
+
+// A marker per warp in one wave; further markers in turn.
+static unsigned marker_grid(int markers) {
+  return (unsigned)std::max(1, std::min((markers + kMarkerWarps - 1) / kMarkerWarps, 8 * 148));
 }
 
 static BinView bin_view(const efsi_bin_plan* P) {
@@ -645,7 +686,7 @@ int efsi_scatter_marker_forces(efsi_bin_plan* P, int32_t marker_count, const flo
   if (marker_count <= 0) return EFSI_OK;
   // 36 bytes per marker (x, F) and 12 per binned particle position read
   EFSI_TIMED(KF_SCATTER, 36.0 * marker_count + 12.0 * P->count_last, s,
-             EFSI_COUNTED k_scatter<<<(marker_count + 7) / 8, 256, 0, s>>>(bin_view(P), marker_count, x_gamma, f_gamma,
+             EFSI_COUNTED k_scatter<<<marker_grid(marker_count), 32 * kMarkerWarps, 0, s>>>(bin_view(P), marker_count, x_gamma, f_gamma,
                                                                              particle_x, external_force,
                                                                              report_device));
   EFSI_LAUNCH_CHECK();
@@ -664,7 +705,7 @@ int efsi_surface_feedback(efsi_bin_plan* P, int32_t marker_count, float* x_gamma
   // 52 bytes per marker (read x; write x, v, n, A) and 40 per binned
   // particle (x, v, normal, area)
   EFSI_TIMED(KF_FEEDBACK, 52.0 * marker_count + 40.0 * P->count_last, s,
-             EFSI_COUNTED k_feedback<<<(marker_count + 7) / 8, 256, 0, s>>>(
+             EFSI_COUNTED k_feedback<<<marker_grid(marker_count), 32 * kMarkerWarps, 0, s>>>(
                  bin_view(P), marker_count, x_gamma, v_gamma, n_gamma, area_gamma, particle_x, particle_v,
                  particle_normal, particle_area, dt, report_device));
   EFSI_LAUNCH_CHECK();

@@ -31,6 +31,7 @@ struct efsi_bin_plan {
   int32_t* offset = nullptr;
   int32_t* cursor = nullptr;
   int32_t* tile_sums = nullptr;  // per-tile bin counts of the offset scan
+  float4* near = nullptr;        // particles in bin order: position and index
 };
 
 namespace efsi {
@@ -198,7 +199,7 @@ struct BinView {
   float R;
   int nb[3];
   int nbins;
-  const int32_t* sorted;
+  const float4* near;
   const int32_t* offset;
 };
 
@@ -318,54 +319,78 @@ __global__ void k_bin_rank(int nbins, const int32_t* offset, const int32_t* in, 
   }
 }
 
+// The particles' positions in bin order, beside their indices: a marker's
+// visits read 16 consecutive bytes a lane where positions behind indices took
+// three scattered loads (96 sectors a warp), which bounded the exchange.
+__global__ void k_near(int P, const int32_t* __restrict__ sorted, const float* __restrict__ x,
+                       float4* __restrict__ near) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= P) return;
+  const int p = sorted[q];
+  near[q] = make_float4(x[3 * p], x[3 * p + 1], x[3 * p + 2], __int_as_float(p));
+}
+
+// x / w with r = 1 / w rounded to nearest: the product corrected by its exact
+// remainder rounds as the quotient does while nothing underflows (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990), and a quotient that does is lost beside the tent's 1.
+__device__ __forceinline__ float div_by(float x, float w, float r) {
+  const float q = __fmul_rn(x, r);
+  const float e = __fmaf_rn(-q, w, x);
+  return fabsf(e) <= 3.402823466e38f ? __fmaf_rn(e, r, q) : q;
+}
+
 // hibm_mpm.py:4838-4848 tent weight.
-__device__ __forceinline__ float tent(const float* xm, const float* xp, float R) {
+__device__ __forceinline__ float tent(const float* xm, float4 xp, float R, float rR) {
+  const float d[3] = {fabsf(xm[0] - xp.x), fabsf(xm[1] - xp.y), fabsf(xm[2] - xp.z)};
   float w = 1.0f;
 #pragma unroll
-  for (int a = 0; a < 3; ++a) w *= fmaxf(1.0f - fabsf(xm[a] - xp[a]) / R, 0.0f);
+  for (int a = 0; a < 3; ++a) w *= fmaxf(1.0f - div_by(d[a], R, rR), 0.0f);
   return w;
 }
 
 // Visits the particles of the 3 x 3 x 3 bins around xm with the whole warp
-// (every lane must call it): lane b < 27 fetches the offsets of neighbour bin
-// b = (d0 + 1) * 9 + (d1 + 1) * 3 + (d2 + 1), a warp scan of the bin sizes
-// numbers the visits 0 .. total-1 in bin order, and the lanes take visits
-// lane, lane + 32, ..., each finding its bin by a binary search over the
-// scan.  The 27 bins are fetched in parallel and every lane has work.
+// (every lane must call it).  The three bins along the last axis lie behind
+// one another, so the neighbourhood is nine runs of particles: lane b < 9
+// fetches the ends of run b = (d0 + 1) * 3 + (d1 + 1), a warp scan of their
+// lengths numbers the visits 0 .. total-1 in bin order, and the lanes take
+// visits lane, lane + 32, ..., each finding its run by a binary search over
+// the scan.  fn gets a particle's position and index.
 template <class Fn>
 __device__ __forceinline__ void for_near(const BinView& B, const float* xm, int lane, Fn fn) {
   int lo = 0, cnt = 0;
-  if (lane < 27) {
-    const int d0 = lane / 9 - 1, d1 = (lane / 3) % 3 - 1, d2 = lane % 3 - 1;
-    const int b0 = bin_axis(xm[0], B.bmin[0], B.invR, B.nb[0]) + d0;
-    const int b1 = bin_axis(xm[1], B.bmin[1], B.invR, B.nb[1]) + d1;
-    const int b2 = bin_axis(xm[2], B.bmin[2], B.invR, B.nb[2]) + d2;
-    if (b0 >= 0 && b0 < B.nb[0] && b1 >= 0 && b1 < B.nb[1] && b2 >= 0 && b2 < B.nb[2]) {
-      const int bin = (b0 * B.nb[1] + b1) * B.nb[2] + b2;
-      lo = __ldg(B.offset + bin);
-      cnt = __ldg(B.offset + bin + 1) - lo;
+  if (lane < 9) {
+    const int b0 = bin_axis(xm[0], B.bmin[0], B.invR, B.nb[0]) + lane / 3 - 1;
+    const int b1 = bin_axis(xm[1], B.bmin[1], B.invR, B.nb[1]) + lane % 3 - 1;
+    const int b2 = bin_axis(xm[2], B.bmin[2], B.invR, B.nb[2]);
+    if (b0 >= 0 && b0 < B.nb[0] && b1 >= 0 && b1 < B.nb[1]) {
+      const int row = (b0 * B.nb[1] + b1) * B.nb[2];
+      lo = __ldg(B.offset + row + max(b2 - 1, 0));
+      cnt = __ldg(B.offset + row + min(b2 + 1, B.nb[2] - 1) + 1) - lo;
     }
   }
   int incl = cnt;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
+  for (int o = 1; o < 16; o <<= 1) {
     const int v = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += v;
   }
-  const int excl = incl - cnt;
-  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  const int excl = lane < 9 ? incl - cnt : 0x7fffffff;
+  const int total = __shfl_sync(0xffffffffu, incl, 8);
   for (int base = 0; base < total; base += 32) {
     const int idx = base + lane;
-    // the last lane j with excl_j <= idx owns visit idx (excl is non-decreasing)
+    // the last run j with excl_j <= idx owns visit idx (excl is non-decreasing)
     int j = 0;
 #pragma unroll
-    for (int step = 16; step > 0; step >>= 1) {
+    for (int step = 8; step > 0; step >>= 1) {
       const int e = __shfl_sync(0xffffffffu, excl, j + step);
       if (e <= idx) j += step;
     }
-    const int lo_j = __shfl_sync(0xffffffffu, lo, j);
-    const int ex_j = __shfl_sync(0xffffffffu, excl, j);
-    if (idx < total) fn(__ldg(B.sorted + lo_j + (idx - ex_j)));
+    const int at = __shfl_sync(0xffffffffu, lo - excl, j);
+    if (idx < total) {
+      const float4 x = __ldg(B.near + at + idx);
+      fn(x, __float_as_int(x.w));
+    }
   }
 }
 
@@ -385,8 +410,8 @@ __device__ __forceinline__ double warp_allsum(double v) {
 // The markers of one block (a warp each, kMarkerWarps at a time) report
 // together: every warp's lane 0 keeps its sums and maxima, and the block adds
 // them once.  With an atomic per marker and value, 65,000 of them on one cache
-// line took most of the exchange of 8,192 markers: the scatter 87 us, the
-// feedback 59; now @SC@ and @FB@.
+// line took most of the exchange of 8,192 markers: the scatter took 87 us, the
+// feedback 59; with one report a block 53 and 47.
 constexpr int kMarkerWarps = 8;
 
 // The larger of two non-negative values by their bits, as atomic_max_nonneg_d
@@ -420,21 +445,21 @@ __device__ __forceinline__ void block_report(const double (&v)[N], unsigned max_
 // warp per marker; the tent-weight sum over the marker's neighbourhood is a
 // warp reduction, then the lanes spread F * w / wsum to the particles.
 __global__ void __launch_bounds__(32 * kMarkerWarps) k_scatter(BinView B, int M, const float* xg, const double* Fg,
-                                                               const float* xp, float* fext, double* rep) {
+                                                               float* fext, double* rep) {
   const int lane = (int)(threadIdx.x & 31);
   double tot[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   for (int m = (int)(blockIdx.x * kMarkerWarps + (threadIdx.x >> 5)); m < M; m += (int)gridDim.x * kMarkerWarps) {
     const float xm[3] = {__ldg(xg + 3 * m), __ldg(xg + 3 * m + 1), __ldg(xg + 3 * m + 2)};
     const double Fm[3] = {__ldg(Fg + 3 * m), __ldg(Fg + 3 * m + 1), __ldg(Fg + 3 * m + 2)};
     const bool valid = finite3(xm) && isfinite(Fm[0]) && isfinite(Fm[1]) && isfinite(Fm[2]);
-    const float R = B.R;
+    const float R = B.R, rR = __frcp_rn(R);
     float wl = 0.0f;
-    if (valid) for_near(B, xm, lane, [&](int p) { wl += tent(xm, xp + 3 * p, R); });
+    if (valid) for_near(B, xm, lane, [&](float4 x, int) { wl += tent(xm, x, R, rR); });
     const float wsum = warp_allsum(wl);
     if (valid && wsum > 1.0e-12f) {
       double e0 = 0, e1 = 0, e2 = 0, contrib = 0;
-      for_near(B, xm, lane, [&](int p) {
-        float w = tent(xm, xp + 3 * p, R);
+      for_near(B, xm, lane, [&](float4 x, int p) {
+        float w = tent(xm, x, R, rR);
         if (w > 0.0f) {
           const double ratio = (double)(w / wsum);
           float f0 = (float)(Fm[0] * ratio), f1 = (float)(Fm[1] * ratio), f2 = (float)(Fm[2] * ratio);
@@ -466,7 +491,7 @@ __global__ void __launch_bounds__(32 * kMarkerWarps) k_scatter(BinView B, int M,
 // tent-weighted sums of particle velocity (and normal / area) as warp
 // reductions.
 __global__ void __launch_bounds__(32 * kMarkerWarps) k_feedback(BinView B, int M, float* xg, float* vg, float* ng,
-                                                                float* Ag, const float* xp, const float* vp,
+                                                                float* Ag, const float* vp,
                                                                 const float* np_, const float* ap, float dt,
                                                                 double* rep) {
   const int lane = (int)(threadIdx.x & 31);
@@ -477,9 +502,9 @@ __global__ void __launch_bounds__(32 * kMarkerWarps) k_feedback(BinView B, int M
     const float no[3] = {ng[3 * m], ng[3 * m + 1], ng[3 * m + 2]};
     const float ao = Ag[m];
     float vs[3] = {0, 0, 0}, ns[3] = {0, 0, 0}, as = 0.0f, ws = 0.0f, gs = 0.0f;
-    const float R = B.R;
-    for_near(B, xo, lane, [&](int p) {
-      float w = tent(xo, xp + 3 * p, R);
+    const float R = B.R, rR = __frcp_rn(R);
+    for_near(B, xo, lane, [&](float4 x, int p) {
+      float w = tent(xo, x, R, rR);
       if (w > 0.0f) {
         vs[0] += w * __ldg(vp + 3 * p);
         vs[1] += w * __ldg(vp + 3 * p + 1);
@@ -562,7 +587,7 @@ static BinView bin_view(const efsi_bin_plan* P) {
   B.invR = P->invR;
   B.R = P->R;
   B.nbins = P->nbins;
-  B.sorted = P->sorted;
+  B.near = P->near;
   B.offset = P->offset;
   return B;
 }
@@ -634,7 +659,8 @@ int efsi_bin_plan_create(int32_t capacity, const float* box_min, const float* bo
       cudaMalloc(&P->count, (P->nbins + 1) * sizeof(int32_t)) != cudaSuccess ||
       cudaMalloc(&P->offset, (P->nbins + 2) * sizeof(int32_t)) != cudaSuccess ||
       cudaMalloc(&P->cursor, (P->nbins + 1) * sizeof(int32_t)) != cudaSuccess ||
-      cudaMalloc(&P->tile_sums, ((P->nbins + 1) / kScanTile + 1) * sizeof(int32_t)) != cudaSuccess) {
+      cudaMalloc(&P->tile_sums, ((P->nbins + 1) / kScanTile + 1) * sizeof(int32_t)) != cudaSuccess ||
+      cudaMalloc(&P->near, capacity * sizeof(float4)) != cudaSuccess) {
     efsi_bin_plan_destroy(P);
     set_error("cudaMalloc failed for the bin plan");
     return EFSI_ERR_CUDA;
@@ -651,6 +677,7 @@ int efsi_bin_plan_destroy(efsi_bin_plan* P) {
   cudaFree(P->offset);
   cudaFree(P->cursor);
   cudaFree(P->tile_sums);
+  cudaFree(P->near);
   delete P;
   return EFSI_OK;
 }
@@ -686,9 +713,10 @@ int efsi_scatter_marker_forces(efsi_bin_plan* P, int32_t marker_count, const flo
   if (marker_count <= 0) return EFSI_OK;
   // 36 bytes per marker (x, F) and 12 per binned particle position read
   EFSI_TIMED(KF_SCATTER, 36.0 * marker_count + 12.0 * P->count_last, s,
-             EFSI_COUNTED k_scatter<<<marker_grid(marker_count), 32 * kMarkerWarps, 0, s>>>(bin_view(P), marker_count, x_gamma, f_gamma,
-                                                                             particle_x, external_force,
-                                                                             report_device));
+             EFSI_COUNTED k_near<<<(unsigned)((P->count_last + 255) / 256), 256, 0, s>>>(P->count_last, P->sorted,
+                                                                                       particle_x, P->near);
+             EFSI_COUNTED k_scatter<<<marker_grid(marker_count), 32 * kMarkerWarps, 0, s>>>(
+                 bin_view(P), marker_count, x_gamma, f_gamma, external_force, report_device));
   EFSI_LAUNCH_CHECK();
   return EFSI_OK;
 }
@@ -705,9 +733,11 @@ int efsi_surface_feedback(efsi_bin_plan* P, int32_t marker_count, float* x_gamma
   // 52 bytes per marker (read x; write x, v, n, A) and 40 per binned
   // particle (x, v, normal, area)
   EFSI_TIMED(KF_FEEDBACK, 52.0 * marker_count + 40.0 * P->count_last, s,
+             EFSI_COUNTED k_near<<<(unsigned)((P->count_last + 255) / 256), 256, 0, s>>>(P->count_last, P->sorted,
+                                                                                       particle_x, P->near);
              EFSI_COUNTED k_feedback<<<marker_grid(marker_count), 32 * kMarkerWarps, 0, s>>>(
-                 bin_view(P), marker_count, x_gamma, v_gamma, n_gamma, area_gamma, particle_x, particle_v,
-                 particle_normal, particle_area, dt, report_device));
+                 bin_view(P), marker_count, x_gamma, v_gamma, n_gamma, area_gamma, particle_v, particle_normal,
+                 particle_area, dt, report_device));
   EFSI_LAUNCH_CHECK();
   return EFSI_OK;
 }

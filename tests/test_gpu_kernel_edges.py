@@ -202,3 +202,99 @@ def test_weight_gradient_boxes(cin, cout, shape):
     xd, gd = x.double(), g.double().reshape(-1, cout)
     ref = torch.stack([gd.T @ _shifted(xd, t).reshape(-1, cin) for t in range(27)], dim=1) + start.double()
     assert _rel(dw.cpu().numpy(), ref.cpu().numpy()) <= 1e-5
+
+
+# ---------------------------------------------------------------------------
+# single-CTA tail of the V-cycle
+# ---------------------------------------------------------------------------
+
+
+@pytest.mark.parametrize("nodes,outlet", [
+    ((7, 6, 9), 0),      # two levels, 60 cells: two warps at the coarsest
+    ((8, 8, 8), 1),      # 64 + 8 cells, one warp
+    ((20, 17, 23), 0),   # 1080 cells: more than one a thread, odd extents
+    ((33, 17, 31), 1),   # 2448 + 360 + 60 cells: the first does not fit beside the others
+])
+def test_vcycle_tail_matches_the_oracle(nodes, outlet):
+    """The tail's rows round as the oracle's (quotients by a corrected
+    reciprocal), so the V-cycle agrees to f64 rounding of the level-0 sweeps,
+    1e-13 as in the general V-cycle test."""
+    from easyfsi_b200.fluid import CartesianFluidSolver, FluidDomainSpec
+
+    grid = _grid(nodes, min(nodes) > 12)
+    fl = CartesianFluidSolver(FluidDomainSpec((0, 0, 0), grid.bounds_max_m, None, 1000.0, 1.0e-3, 1.0e-3,
+                                              cartesian_grid=grid))
+    ofl = orc.OracleFluid(grid, rho=1000.0, mu=1.0e-3)
+    rng = np.random.default_rng(nodes[0])
+    obs = (rng.random(nodes) < 0.03).astype(np.int32)
+    fl.obstacle.from_numpy(obs)
+    ofl.obstacle[...] = obs
+    r = rng.normal(size=nodes) * (obs == 0)
+    fl.cg_r.from_numpy(r)
+    fl._apply_fv_multigrid_preconditioner(fl.cg_r, pressure_outlet_zmin=bool(outlet))
+    assert _rel(fl.cg_z.to_numpy(), ofl.vcycle(r, outlet)) <= 1e-13
+
+
+# ---------------------------------------------------------------------------
+# particle binning
+# ---------------------------------------------------------------------------
+
+
+@pytest.mark.parametrize("nodes", [(8, 8, 8), (80, 84, 76), (84, 84, 84)])
+def test_substep_over_many_tiles_conserves_mass_and_momentum(nodes):
+    """Tile counts on both sides of one scan block's 8192 entries: particles in
+    the first, middle and last tiles all reach the grid, so the reported mass
+    and momentum are the particles' (f32 products, f64 sums: 1e-6)."""
+    from easyfsi_b200.neo_hookean_mpm import NeoHookeanMpmState
+
+    rng = np.random.default_rng(nodes[1])
+    lo, hi = 3.0 / np.asarray(nodes), 1.0 - 3.0 / np.asarray(nodes)
+    x = np.concatenate([lo + 0.02 * rng.random((40, 3)), 0.4 + 0.2 * rng.random((40, 3)), hi - 0.02 * rng.random((40, 3))])
+    v = rng.normal(size=x.shape).astype(np.float32) * 0.01
+    n = len(x)
+    so = NeoHookeanMpmState(particle_capacity=n, bounds_min_m=(0, 0, 0), bounds_max_m=(1, 1, 1), grid_nodes=nodes)
+    so.load_particles(positions_m=x.astype(np.float32), volumes_m3=np.full(n, 1e-6, np.float32),
+                      masses_kg=np.full(n, 1e-3, np.float32), region_ids=np.full(n, 1, np.int32),
+                      normals=np.zeros((n, 3), np.float32), areas_m2=np.zeros(n, np.float32))
+    so.v.from_numpy(np.concatenate([v, np.zeros((so.v.tensor.shape[0] - n, 3), np.float32)]))
+    so.step(dt_s=1.0e-6, mu_pa=1.0e4, lambda_pa=1.0e4, primary_region_id=1, secondary_region_id=2,
+            velocity_damping=1.0, read_report=False)
+    got = so.v.to_numpy()[:n]
+    # nearly stress-free particles exchange momentum only with their neighbours
+    np.testing.assert_allclose(got.sum(0), v.sum(0), rtol=0.0, atol=1e-6 * np.abs(v).sum())
+
+
+# ---------------------------------------------------------------------------
+# projection reports
+# ---------------------------------------------------------------------------
+
+
+@pytest.mark.parametrize("nodes", [(5, 4, 7), (12, 9, 33), (40, 50, 60)])
+def test_dirichlet_row_report_sums(nodes):
+    """Row count, sum and maximum of |dv| against float64 sums of the same f32
+    values; the square root rounds to f32, so 1e-6."""
+    from easyfsi_b200.fluid import CartesianFluidSolver, FluidDomainSpec
+
+    grid = _grid(nodes, False)
+    fl = CartesianFluidSolver(FluidDomainSpec((0, 0, 0), grid.bounds_max_m, None, 1000.0, 1.0e-3, 1.0e-3,
+                                              cartesian_grid=grid))
+    rng = np.random.default_rng(nodes[0])
+    obs = (rng.random(nodes) < 0.1).astype(np.int32)
+    act = (rng.random(nodes) < 0.3).astype(np.int32)
+    vel, val = (rng.normal(size=nodes + (3,)).astype(np.float32) for _ in range(2))
+    fl.obstacle.from_numpy(obs)
+    fl.velocity_dirichlet_boundary_active.from_numpy(act)
+    fl.velocity_dirichlet_boundary_value_mps.from_numpy(val)
+    fl.velocity_dirichlet_boundary_projection_weight.from_numpy(np.ones(nodes, np.float32))
+    fl.velocity.from_numpy(vel)
+    rep = fl.apply_velocity_dirichlet_boundary_rows()
+    rows = (act != 0) & (obs == 0)
+    d = np.linalg.norm((val - vel).astype(np.float64)[rows], axis=1)
+    h = [1.0 / m for m in nodes]
+    impulse = 1000.0 * h[0] * h[1] * h[2] * (val - vel).astype(np.float64)[rows].sum(0)
+    assert rep.active_cells == rows.sum()
+    assert rep.max_delta_mps == pytest.approx(d.max(), rel=1e-6)
+    assert rep.mean_delta_mps == pytest.approx(d.mean(), rel=1e-6)
+    np.testing.assert_allclose(rep.momentum_delta_n_s, impulse, rtol=0.0,
+                               atol=1e-6 * 1000.0 * h[0] * h[1] * h[2] * d.sum())
+    np.testing.assert_array_equal(fl.velocity.to_numpy()[rows], val[rows])

@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(kCThreads, 4)
              const __grid_constant__ CUtensorMap map_d, const __grid_constant__ CUtensorMap map_rd,
              TV* __restrict__ out, double* __restrict__ out64, int outlet, double omega, ProlongSrc pr,
              double* partials, CgScalars* sc) {
-  pdl_wait();
+  pdl_wait_early();
   using Op = ColumnSweep<TV, kProlong, kAux, kDots>;
   ColumnGeom g;
   const bool any = column_geom(L, chunk, g);
@@ -805,7 +805,7 @@ __global__ void __launch_bounds__(kCThreads, 4)
     kc_restrict(LevelDev F, int chunk, const __grid_constant__ CUtensorMap map_p,
                 const __grid_constant__ CUtensorMap map_r, const __grid_constant__ CUtensorMap map_m, int outlet,
                 LevelDev C, float* __restrict__ crhs, float* __restrict__ cpa, double omega, CgScalars* sc) {
-  pdl_wait();
+  pdl_wait_early();
   ColumnGeom g;
   const bool any = column_geom(F, chunk, g);
   ColumnRestrict<TV, kAux> op{F, g, outlet, C, crhs, cpa, omega};

@@ -179,7 +179,7 @@ template <typename TP, bool kNegR, bool kZero>
 __global__ void __launch_bounds__(256) k_sweep(LevelDev L, const TP* __restrict__ p, const void* rhs,
                                                TP* __restrict__ out, int outlet, double omega, ProlongSrc pr,
                                                double* partials, CgScalars* sc) {
-  pdl_wait();
+  pdl_wait_early();
   EFSI_CELL_PROLOGUE(L)
   double zv = 0.0;
   if (active) {
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(256) k_residual(LevelDev L, const TP* __restri
 template <typename TP, bool kNegR, bool kFromP>
 __global__ void __launch_bounds__(256) k_restrict(LevelDev F, const TP* __restrict__ p_or_res, const void* rhs,
                                                   int outlet, int cnx, int cny, int cnz, float* __restrict__ crhs) {
-  pdl_wait();
+  pdl_wait_early();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int i = blockIdx.z * blockDim.z + threadIdx.z;
@@ -393,7 +393,7 @@ template <typename TP, bool kNegR, bool kZero>
 __global__ void __launch_bounds__(256) kt_sweep(LevelDev L, const TP* __restrict__ p, const void* rhs,
                                                 TP* __restrict__ out, int outlet, double omega, ProlongSrc pr,
                                                 double* partials, CgScalars* sc) {
-  pdl_wait();
+  pdl_wait_early();
   const int nt = tiles_of(L.nx, L.ny, L.nz);
   const int64_t sx = (int64_t)L.ny * L.nz;
   double zsum = 0.0;
@@ -1058,7 +1058,7 @@ __global__ void __launch_bounds__(kTailThreads) k_mg_tail(TailDesc T) {
   // started after everything before it was complete, the tables' inputs
   // included, and writes none of them.
   tail_prologue(T, tail_smem);
-  pdl_wait();
+  pdl_wait_early();
   tail_body(T, tail_smem);
 }
 

@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(kMK* kTY, 3)
              const __grid_constant__ CUtensorMap map_r, const __grid_constant__ CUtensorMap map_m,
              TP* __restrict__ out, int outlet, double omega, ProlongSrc pr, double* partials, CgScalars* sc,
              const double* __restrict__ delta, const double* __restrict__ rden) {
-  pdl_wait();
+  pdl_wait_early();
   using TR = typename std::conditional<kNegR, double, TP>::type;
   MarchGeom g;
   const bool any = march_geom(L, chunk, g);
@@ -662,7 +662,7 @@ __global__ void __launch_bounds__(kMK* kTY, 3)
                const __grid_constant__ CUtensorMap map_r, const __grid_constant__ CUtensorMap map_m,
                float* __restrict__ out, double* __restrict__ out64, int outlet, double omega, ProlongSrc pr,
                double* partials, CgScalars* sc, const double* __restrict__ delta) {
-  pdl_wait();
+  pdl_wait_early();
   MarchGeom g;
   const bool any = march_geom(L, chunk, g);
   Sweep32Op<kProlong, kAux, kDots> op{{L, out, outlet, omega, pr, partials != nullptr, 0.0, delta, 0.0, 0.0, 0.0, 0.0},
@@ -688,7 +688,7 @@ template <typename TP, bool kNegR, bool kAux>
 __global__ void __launch_bounds__(kMK* kTY)
     km_sweep0(LevelDev L, const void* rhs, TP* __restrict__ out, int outlet, double omega, double* partials,
               CgScalars* sc, const double* __restrict__ rden) {
-  pdl_wait();
+  pdl_wait_early();
   const int k = (int)(blockIdx.x * kMK + threadIdx.x), j = (int)(blockIdx.y * kTY + threadIdx.y);
   const int i0 = (int)blockIdx.z * kSweep0Planes;
   double zsum = 0.0;
@@ -970,7 +970,7 @@ __global__ void __launch_bounds__(kMK* kTY, 3)
                 const __grid_constant__ CUtensorMap map_r, const __grid_constant__ CUtensorMap map_m, int outlet,
                 int cnx, int cny, int cnz, float* __restrict__ crhs, CgScalars* sc, LevelDev C,
                 float* __restrict__ cpa, double omega) {
-  pdl_wait();
+  pdl_wait_early();
   using TR = typename std::conditional<kNegR, double, TP>::type;
   __shared__ double rs[2][kMJ * kMK];
   __shared__ unsigned char rsolid[2][kMJ * kMK];

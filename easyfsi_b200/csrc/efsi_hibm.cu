@@ -31,7 +31,6 @@ struct efsi_bin_plan {
   int32_t* offset = nullptr;
   int32_t* cursor = nullptr;
   int32_t* tile_sums = nullptr;  // per-tile bin counts of the offset scan
-  float4* near = nullptr;        // particles in bin order: position and index
 };
 
 namespace efsi {
@@ -199,7 +198,7 @@ struct BinView {
   float R;
   int nb[3];
   int nbins;
-  const float4* near;
+  const int32_t* sorted;
   const int32_t* offset;
 };
 
@@ -319,17 +318,6 @@ __global__ void k_bin_rank(int nbins, const int32_t* offset, const int32_t* in, 
   }
 }
 
-// The particles' positions in bin order, beside their indices: a marker's
-// visits read 16 consecutive bytes a lane where positions behind indices took
-// three scattered loads (96 sectors a warp), which bounded the exchange.
-__global__ void k_near(int P, const int32_t* __restrict__ sorted, const float* __restrict__ x,
-                       float4* __restrict__ near) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= P) return;
-  const int p = sorted[q];
-  near[q] = make_float4(x[3 * p], x[3 * p + 1], x[3 * p + 2], __int_as_float(p));
-}
-
 // x / w with r = 1 / w rounded to nearest: the product corrected by its exact
 // remainder rounds as the quotient does while nothing underflows (Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000
@@ -341,11 +329,10 @@ __device__ __forceinline__ float div_by(float x, float w, float r) {
 }
 
 // hibm_mpm.py:4838-4848 tent weight.
-__device__ __forceinline__ float tent(const float* xm, float4 xp, float R, float rR) {
-  const float d[3] = {fabsf(xm[0] - xp.x), fabsf(xm[1] - xp.y), fabsf(xm[2] - xp.z)};
+__device__ __forceinline__ float tent(const float* xm, const float* xp, float R, float rR) {
   float w = 1.0f;
 #pragma unroll
-  for (int a = 0; a < 3; ++a) w *= fmaxf(1.0f - div_by(d[a], R, rR), 0.0f);
+  for (int a = 0; a < 3; ++a) w *= fmaxf(1.0f - div_by(fabsf(xm[a] - xp[a]), R, rR), 0.0f);
   return w;
 }
 
@@ -355,7 +342,9 @@ __device__ __forceinline__ float tent(const float* xm, float4 xp, float R, float
 // fetches the ends of run b = (d0 + 1) * 3 + (d1 + 1), a warp scan of their
 // lengths numbers the visits 0 .. total-1 in bin order, and the lanes take
 // visits lane, lane + 32, ..., each finding its run by a binary search over
-// the scan.  fn gets a particle's position and index.
+// the scan.  fn gets a particle's index.  Only the bins' own entries of
+// `sorted` are visited: those of the bucket of non-finite particles behind
+// them are not kept in order.
 template <class Fn>
 __device__ __forceinline__ void for_near(const BinView& B, const float* xm, int lane, Fn fn) {
   int lo = 0, cnt = 0;
@@ -387,10 +376,7 @@ __device__ __forceinline__ void for_near(const BinView& B, const float* xm, int 
       if (e <= idx) j += step;
     }
     const int at = __shfl_sync(0xffffffffu, lo - excl, j);
-    if (idx < total) {
-      const float4 x = __ldg(B.near + at + idx);
-      fn(x, __float_as_int(x.w));
-    }
+    if (idx < total) fn(__ldg(B.sorted + at + idx));
   }
 }
 
@@ -445,7 +431,8 @@ __device__ __forceinline__ void block_report(const double (&v)[N], unsigned max_
 // warp per marker; the tent-weight sum over the marker's neighbourhood is a
 // warp reduction, then the lanes spread F * w / wsum to the particles.
 __global__ void __launch_bounds__(32 * kMarkerWarps) k_scatter(BinView B, int M, const float* xg, const double* Fg,
-                                                               float* fext, double* rep) {
+                                                               const float* xp, float* fext,
+                                                               double* rep) {
   const int lane = (int)(threadIdx.x & 31);
   double tot[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   for (int m = (int)(blockIdx.x * kMarkerWarps + (threadIdx.x >> 5)); m < M; m += (int)gridDim.x * kMarkerWarps) {
@@ -454,12 +441,12 @@ __global__ void __launch_bounds__(32 * kMarkerWarps) k_scatter(BinView B, int M,
     const bool valid = finite3(xm) && isfinite(Fm[0]) && isfinite(Fm[1]) && isfinite(Fm[2]);
     const float R = B.R, rR = __frcp_rn(R);
     float wl = 0.0f;
-    if (valid) for_near(B, xm, lane, [&](float4 x, int) { wl += tent(xm, x, R, rR); });
+    if (valid) for_near(B, xm, lane, [&](int p) { wl += tent(xm, xp + 3 * p, R, rR); });
     const float wsum = warp_allsum(wl);
     if (valid && wsum > 1.0e-12f) {
       double e0 = 0, e1 = 0, e2 = 0, contrib = 0;
-      for_near(B, xm, lane, [&](float4 x, int p) {
-        float w = tent(xm, x, R, rR);
+      for_near(B, xm, lane, [&](int p) {
+        float w = tent(xm, xp + 3 * p, R, rR);
         if (w > 0.0f) {
           const double ratio = (double)(w / wsum);
           float f0 = (float)(Fm[0] * ratio), f1 = (float)(Fm[1] * ratio), f2 = (float)(Fm[2] * ratio);
@@ -491,7 +478,7 @@ __global__ void __launch_bounds__(32 * kMarkerWarps) k_scatter(BinView B, int M,
 // tent-weighted sums of particle velocity (and normal / area) as warp
 // reductions.
 __global__ void __launch_bounds__(32 * kMarkerWarps) k_feedback(BinView B, int M, float* xg, float* vg, float* ng,
-                                                                float* Ag, const float* vp,
+                                                                float* Ag, const float* xp, const float* vp,
                                                                 const float* np_, const float* ap, float dt,
                                                                 double* rep) {
   const int lane = (int)(threadIdx.x & 31);
@@ -503,8 +490,8 @@ __global__ void __launch_bounds__(32 * kMarkerWarps) k_feedback(BinView B, int M
     const float ao = Ag[m];
     float vs[3] = {0, 0, 0}, ns[3] = {0, 0, 0}, as = 0.0f, ws = 0.0f, gs = 0.0f;
     const float R = B.R, rR = __frcp_rn(R);
-    for_near(B, xo, lane, [&](float4 x, int p) {
-      float w = tent(xo, x, R, rR);
+    for_near(B, xo, lane, [&](int p) {
+      float w = tent(xo, xp + 3 * p, R, rR);
       if (w > 0.0f) {
         vs[0] += w * __ldg(vp + 3 * p);
         vs[1] += w * __ldg(vp + 3 * p + 1);
@@ -587,7 +574,7 @@ static BinView bin_view(const efsi_bin_plan* P) {
   B.invR = P->invR;
   B.R = P->R;
   B.nbins = P->nbins;
-  B.near = P->near;
+  B.sorted = P->sorted;
   B.offset = P->offset;
   return B;
 }
@@ -659,8 +646,7 @@ int efsi_bin_plan_create(int32_t capacity, const float* box_min, const float* bo
       cudaMalloc(&P->count, (P->nbins + 1) * sizeof(int32_t)) != cudaSuccess ||
       cudaMalloc(&P->offset, (P->nbins + 2) * sizeof(int32_t)) != cudaSuccess ||
       cudaMalloc(&P->cursor, (P->nbins + 1) * sizeof(int32_t)) != cudaSuccess ||
-      cudaMalloc(&P->tile_sums, ((P->nbins + 1) / kScanTile + 1) * sizeof(int32_t)) != cudaSuccess ||
-      cudaMalloc(&P->near, capacity * sizeof(float4)) != cudaSuccess) {
+      cudaMalloc(&P->tile_sums, ((P->nbins + 1) / kScanTile + 1) * sizeof(int32_t)) != cudaSuccess) {
     efsi_bin_plan_destroy(P);
     set_error("cudaMalloc failed for the bin plan");
     return EFSI_ERR_CUDA;
@@ -677,7 +663,6 @@ int efsi_bin_plan_destroy(efsi_bin_plan* P) {
   cudaFree(P->offset);
   cudaFree(P->cursor);
   cudaFree(P->tile_sums);
-  cudaFree(P->near);
   delete P;
   return EFSI_OK;
 }
@@ -713,10 +698,8 @@ int efsi_scatter_marker_forces(efsi_bin_plan* P, int32_t marker_count, const flo
   if (marker_count <= 0) return EFSI_OK;
   // 36 bytes per marker (x, F) and 12 per binned particle position read
   EFSI_TIMED(KF_SCATTER, 36.0 * marker_count + 12.0 * P->count_last, s,
-             EFSI_COUNTED k_near<<<(unsigned)((P->count_last + 255) / 256), 256, 0, s>>>(P->count_last, P->sorted,
-                                                                                       particle_x, P->near);
              EFSI_COUNTED k_scatter<<<marker_grid(marker_count), 32 * kMarkerWarps, 0, s>>>(
-                 bin_view(P), marker_count, x_gamma, f_gamma, external_force, report_device));
+                 bin_view(P), marker_count, x_gamma, f_gamma, particle_x, external_force, report_device));
   EFSI_LAUNCH_CHECK();
   return EFSI_OK;
 }
@@ -733,11 +716,9 @@ int efsi_surface_feedback(efsi_bin_plan* P, int32_t marker_count, float* x_gamma
   // 52 bytes per marker (read x; write x, v, n, A) and 40 per binned
   // particle (x, v, normal, area)
   EFSI_TIMED(KF_FEEDBACK, 52.0 * marker_count + 40.0 * P->count_last, s,
-             EFSI_COUNTED k_near<<<(unsigned)((P->count_last + 255) / 256), 256, 0, s>>>(P->count_last, P->sorted,
-                                                                                       particle_x, P->near);
              EFSI_COUNTED k_feedback<<<marker_grid(marker_count), 32 * kMarkerWarps, 0, s>>>(
-                 bin_view(P), marker_count, x_gamma, v_gamma, n_gamma, area_gamma, particle_v, particle_normal,
-                 particle_area, dt, report_device));
+                 bin_view(P), marker_count, x_gamma, v_gamma, n_gamma, area_gamma, particle_x, particle_v,
+                 particle_normal, particle_area, dt, report_device));
   EFSI_LAUNCH_CHECK();
   return EFSI_OK;
 }

@@ -265,6 +265,57 @@ def test_substep_over_many_tiles_conserves_mass_and_momentum(nodes):
 
 
 # ---------------------------------------------------------------------------
+# marker exchange
+# ---------------------------------------------------------------------------
+
+
+def _exchange(x, v, normal, area, marker_x, marker_f, radius):
+    """Force on the particles, the markers after the feedback, and both reports."""
+    from easyfsi_b200.hibm_mpm import HibmMpmSurfaceMarkers
+
+    m = len(marker_x)
+    mk = HibmMpmSurfaceMarkers(marker_capacity=m)
+    mk.load_markers(positions_m=marker_x.tolist(), velocities_mps=np.zeros_like(marker_x).tolist(),
+                    normals=[(0.0, 0.0, 1.0)] * m, areas_m2=[1.0] * m, region_ids=[1] * m)
+    mk.F_gamma_n.from_numpy(marker_f)
+    xt, vt, nt, at = (torch.from_numpy(q).cuda() for q in (x, v, normal, area))
+    force = torch.zeros_like(xt)
+    scatter = mk.scatter_marker_forces_to_mpm_particles(force, xt, particle_count=len(x), support_radius_m=radius)
+    feedback = mk.update_surface_feedback_from_mpm_surface_particles(xt, vt, nt, at, particle_count=len(x),
+                                                                     support_radius_m=radius, dt_s=1.0e-3)
+    state = [f.to_numpy() for f in (mk.x_gamma_m, mk.v_gamma_mps, mk.n_gamma, mk.A_gamma_m2)]
+    return force.cpu().numpy(), state, scatter, feedback
+
+
+@pytest.mark.parametrize("count,radius", [(500, 0.02), (3000, 0.3)])  # more bins than particles, and fewer
+def test_marker_exchange_ignores_particles_that_are_not_finite(count, radius):
+    """Particles with NaN or infinite positions among others: markers, reports
+    and forces are those of the finite particles alone.  The feedback sums the
+    same values in the same order; the forces are f32 atomic sums of at most 60
+    contributions, 60 x 2^-24 of the sum of their sizes."""
+    rng = np.random.default_rng(count)
+    x = rng.random((count, 3)).astype(np.float32)
+    v, normal = (rng.normal(size=(count, 3)).astype(np.float32) for _ in range(2))
+    area = rng.random(count).astype(np.float32)
+    marker_x = (x[:60] + 0.3 * radius * rng.uniform(-1.0, 1.0, (60, 3))).astype(np.float32)
+    marker_f = rng.normal(size=(60, 3))
+    bad = np.concatenate([[0, count - 1], rng.choice(np.arange(100, count - 1), 20, replace=False)])
+    x[bad, np.arange(len(bad)) % 3] = np.resize([np.nan, np.inf, -np.inf], len(bad))
+    good = np.setdiff1d(np.arange(count), bad)
+    force, state, scatter, feedback = _exchange(x, v, normal, area, marker_x, marker_f, radius)
+    ref_force, ref_state, ref_scatter, ref_feedback = _exchange(x[good], v[good], normal[good], area[good], marker_x,
+                                                                marker_f, radius)
+    assert scatter.active_marker_count >= 40
+    for got, ref in zip(state, ref_state):
+        np.testing.assert_array_equal(got, ref)
+    assert feedback == ref_feedback
+    assert (scatter.active_marker_count, scatter.invalid_marker_count, scatter.active_particle_count) == (
+        ref_scatter.active_marker_count, ref_scatter.invalid_marker_count, ref_scatter.active_particle_count)
+    assert not force[bad].any()
+    np.testing.assert_allclose(force[good], ref_force, rtol=0.0, atol=60 * 2.0**-24 * np.abs(marker_f).sum(0).max())
+
+
+# ---------------------------------------------------------------------------
 # projection reports
 # ---------------------------------------------------------------------------
 

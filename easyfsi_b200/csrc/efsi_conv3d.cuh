@@ -180,7 +180,21 @@ __host__ __device__ inline uint32_t tmem_columns(int n) {
   return c;
 }
 
+// Eight channels, or zeros: with kVec one 16-byte asynchronous copy, which
+// needs an aligned source, otherwise a load per element.
+template <bool kVec>
+__device__ __forceinline__ void copy8(void* dst, const __nv_bfloat16* src, bool ok) {
+  if (kVec) {
+    cp_async16(dst, src, ok ? 16 : 0);
+  } else {
+    __align__(16) __nv_bfloat16 v[8];
+    for (int q = 0; q < 8; ++q) v[q] = ok ? src[q] : __float2bfloat16_rn(0.0f);
+    *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(v);
+  }
+}
+
 // 16-byte chunk c of voxel (i, j, k), or zeros outside the volume.
+template <bool kVec>
 __device__ __forceinline__ void copy_chunk(unsigned char* dst, const ConvInput& in, int nx, int ny, int nz, int cin,
                                            int i, int j, int k, int c) {
   const bool ok = i >= 0 && i < nx && j >= 0 && j < ny && k >= 0 && k < nz;
@@ -192,7 +206,7 @@ __device__ __forceinline__ void copy_chunk(unsigned char* dst, const ConvInput& 
     else
       src = in.x + (((int64_t)i * ny + j) * nz + k) * (cin - in.ca) + (c * 8 - in.ca);
   }
-  cp_async16(dst, src, ok ? 16 : 0);
+  copy8<kVec>(dst, src, ok);
 }
 
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
@@ -236,7 +250,7 @@ __global__ void __launch_bounds__(kThreads) k_conv3d_tc(ConvArgs A, ConvTile T) 
     for (int e = tid; e < rows * kch; e += kThreads) {
       const int row = e / kch, c = e - row * kch;
       const int line = row / zp, z = row - line * zp;
-      copy_chunk(dst + c * T.cs + row * 16, A.in, A.nx, A.ny, A.nz, cin, p, j0 - 1 + line, z0 - 1 + z, c);
+      copy_chunk<true>(dst + c * T.cs + row * 16, A.in, A.nx, A.ny, A.nz, cin, p, j0 - 1 + line, z0 - 1 + z, c);
     }
   };
   for (int q = tid; q < 27 * nt * kch; q += kThreads) {
@@ -367,6 +381,9 @@ struct WgradTile {
   unsigned cols;
 };
 
+// kVec: x and dy start on 16-byte boundaries (their rows are multiples of 32
+// bytes); they may start at any element otherwise.
+template <bool kVec>
 __global__ void __launch_bounds__(kThreads) k_wgrad_tc(WgradArgs A, WgradTile T) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar;
@@ -408,15 +425,15 @@ __global__ void __launch_bounds__(kThreads) k_wgrad_tc(WgradArgs A, WgradTile T)
     for (int e = tid; e < T.rows * (g1 - g0); e += kThreads) {
       const int row = e / (g1 - g0), g = g0 + e - row * (g1 - g0);
       const int line = row / zp, z = row - line * zp, di = g / kch - 1, c = g % kch;
-      copy_chunk(sx + (g - g0) * T.cs + row * 16, A.in, A.nx, A.ny, A.nz, cin, i + di,
+      copy_chunk<kVec>(sx + (g - g0) * T.cs + row * 16, A.in, A.nx, A.ny, A.nz, cin, i + di,
                  line < T.bj ? j0 + line + dj : -1, z0 - 1 + z, c);
     }
     for (int e = tid; e < T.rows * nch; e += kThreads) {
       const int row = e / nch, c = e - row * nch;
       const int line = row / zp, z = row - line * zp, j = j0 + line, k = z0 - 1 + z;
       const bool in = line < T.bj && z >= 1 && z <= T.bz && j < A.ny && k < A.nz;
-      cp_async16(sd + c * T.ds + row * 16,
-                 in ? A.dy + (((int64_t)i * A.ny + j) * A.nz + k) * A.cout + n0 + c * 8 : A.dy, in ? 16 : 0);
+      copy8<kVec>(sd + c * T.ds + row * 16,
+                  in ? A.dy + (((int64_t)i * A.ny + j) * A.nz + k) * A.cout + n0 + c * 8 : A.dy, in);
     }
     cp_async_commit();
     cp_async_wait<0>();

@@ -404,7 +404,7 @@ int set_kernel_attributes() {
   EFSI_CUDA_CHECK(
       cudaFuncSetAttribute(conv::k_conv3d_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, conv::kMaxSmem));
   EFSI_CUDA_CHECK(
-      cudaFuncSetAttribute(conv::k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, conv::kMaxSmem));
+      cudaFuncSetAttribute(conv::k_wgrad_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, conv::kMaxSmem));
   done = true;
   return EFSI_OK;
 }
@@ -425,7 +425,15 @@ int wgrad_launch(const conv::WgradTile& T, const Dims& d, int cin, int cout, con
   const unsigned gy = 3u * (unsigned)(3 / T.ndk), gz = (unsigned)(T.nmb * (cout / T.nt));
   // two CTAs per SM take the boxes in turn; each adds its sums once
   const unsigned gx = (unsigned)std::min<int64_t>(T.items, std::max<int64_t>(1, 2 * 148 / (int64_t)(gy * gz)));
-  EFSI_COUNTED conv::k_wgrad_tc<<<dim3(gx, gy, gz), conv::kThreads, T.smem, s>>>(A, T);
+  const uintptr_t at = reinterpret_cast<uintptr_t>(in.x) | reinterpret_cast<uintptr_t>(in.coarse) |
+                       reinterpret_cast<uintptr_t>(dpre);
+  if ((at & 15u) == 0) {
+    EFSI_COUNTED conv::k_wgrad_tc<true><<<dim3(gx, gy, gz), conv::kThreads, T.smem, s>>>(A, T);
+  } else {
+    EFSI_CUDA_CHECK(
+        cudaFuncSetAttribute(conv::k_wgrad_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, conv::kMaxSmem));
+    EFSI_COUNTED conv::k_wgrad_tc<false><<<dim3(gx, gy, gz), conv::kThreads, T.smem, s>>>(A, T);
+  }
   return EFSI_OK;
 }
 

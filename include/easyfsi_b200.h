@@ -732,13 +732,14 @@ typedef struct efsi_unet efsi_unet;
 /* One 3x3x3 convolution, zero padded, of x (BF16 [n][cin]) with w (BF16
  * [cout][27][cin], tap t = (di + 1) * 9 + (dj + 1) * 3 + (dk + 1)), plus the
  * bias and an optional ReLU; writes BF16 y [n][cout] and/or FP32 yf.  cin and
- * cout are multiples of 16.  A pipeline wait that gives up sets
- * *error_device. */
+ * cout are multiples of 16; x, w, y and yf start on 16-byte boundaries.  A
+ * pipeline wait that gives up sets *error_device. */
 int efsi_conv3d_bf16(int32_t nx, int32_t ny, int32_t nz, int32_t cin, int32_t cout, const void* x, const void* w,
                      const float* bias, int32_t relu, void* y, float* yf, int32_t* error_device, void* stream);
 
 /* Weight gradient of that convolution: dw[co][t][ci] += sum_v dy[v][co]
- * x[v + off(t)][ci] (FP32 accumulation into dw). */
+ * x[v + off(t)][ci] (FP32 accumulation into dw).  x and dy may start at any
+ * BF16 element; on 16-byte boundaries they are copied faster. */
 int efsi_conv3d_wgrad(int32_t nx, int32_t ny, int32_t nz, int32_t cin, int32_t cout, const void* x,
                       const void* dy, float* dw, void* stream);
 

@@ -184,24 +184,53 @@ def test_convolution_boxes(cin, cout, shape):
     assert torch.equal(yb, yf.to(torch.bfloat16))
 
 
+def _weight_gradient(x, g, start):
+    from easyfsi_b200 import _native
+
+    dw = start.clone()
+    _native.call("efsi_conv3d_wgrad", *x.shape[:3], x.shape[3], g.shape[3], x.data_ptr(), g.data_ptr(), dw.data_ptr(),
+                 torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    return dw
+
+
+def _weight_gradient_reference(x, g, start):
+    xd, gd = x.double(), g.double().reshape(-1, g.shape[3])
+    return torch.stack([gd.T @ _shifted(xd, t).reshape(-1, x.shape[3]) for t in range(27)], dim=1) + start.double()
+
+
 @pytest.mark.parametrize("cin,cout,shape", [c for c in CONV_SHAPES if c[0] * c[1] <= 7168] + [
     (448, 16, (2, 2, 9)), (16, 448, (3, 4, 17)), (16, 16, (40, 33, 31))])
 def test_weight_gradient_boxes(cin, cout, shape):
     """Boxes of a plane, several M blocks and channel splits; FP32 sums over
     the voxels against float64, added to what is there."""
-    from easyfsi_b200 import _native
-
     gen = torch.Generator(device="cuda")
     gen.manual_seed(cin * 1000 + cout + 1)
     x, g = _volume(shape, cin, gen), _volume(shape, cout, gen)
     start = torch.randn((cout, 27, cin), generator=gen, device="cuda")
-    dw = start.clone()
-    _native.call("efsi_conv3d_wgrad", *shape, cin, cout, x.data_ptr(), g.data_ptr(), dw.data_ptr(),
-                 torch.cuda.current_stream().cuda_stream)
-    torch.cuda.synchronize()
-    xd, gd = x.double(), g.double().reshape(-1, cout)
-    ref = torch.stack([gd.T @ _shifted(xd, t).reshape(-1, cin) for t in range(27)], dim=1) + start.double()
-    assert _rel(dw.cpu().numpy(), ref.cpu().numpy()) <= 1e-5
+    dw = _weight_gradient(x, g, start)
+    assert _rel(dw.cpu().numpy(), _weight_gradient_reference(x, g, start).cpu().numpy()) <= 1e-5
+
+
+@pytest.mark.parametrize("x_off,g_off", [(1, 0), (0, 3), (4, 8), (8, 5)])  # elements past a 16-byte boundary
+def test_weight_gradient_of_operands_at_any_element(x_off, g_off):
+    """Operands that do not start on a 16-byte boundary: the same gradient, to
+    the same bound as the aligned ones."""
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(10 * x_off + g_off)
+    shape, cin, cout = (3, 9, 34), 48, 32
+
+    def at(t, off):
+        buf = torch.empty(t.numel() + 16, dtype=t.dtype, device="cuda")
+        view = buf[off : off + t.numel()].view(t.shape)
+        view.copy_(t)
+        return view
+
+    x, g = at(_volume(shape, cin, gen), x_off), at(_volume(shape, cout, gen), g_off)
+    assert x.data_ptr() % 16 == 2 * x_off % 16 and g.data_ptr() % 16 == 2 * g_off % 16
+    start = torch.randn((cout, 27, cin), generator=gen, device="cuda")
+    dw = _weight_gradient(x, g, start)
+    assert _rel(dw.cpu().numpy(), _weight_gradient_reference(x, g, start).cpu().numpy()) <= 1e-5
 
 
 # ---------------------------------------------------------------------------

@@ -193,20 +193,24 @@ __device__ __forceinline__ void copy8(void* dst, const __nv_bfloat16* src, bool 
   }
 }
 
+__device__ __forceinline__ bool in_volume(int nx, int ny, int nz, int i, int j, int k) {
+  return i >= 0 && i < nx && j >= 0 && j < ny && k >= 0 && k < nz;
+}
+
+// Channel ch of voxel (i, j, k) of the volume.
+__device__ __forceinline__ const __nv_bfloat16* channel_at(const ConvInput& in, int ny, int nz, int cin, int i, int j,
+                                                           int k, int ch) {
+  if (ch < in.ca)
+    return in.coarse + (((int64_t)(i >> 1) * ((ny + 1) >> 1) + (j >> 1)) * ((nz + 1) >> 1) + (k >> 1)) * in.ca + ch;
+  return in.x + (((int64_t)i * ny + j) * nz + k) * (cin - in.ca) + (ch - in.ca);
+}
+
 // 16-byte chunk c of voxel (i, j, k), or zeros outside the volume.
 template <bool kVec>
 __device__ __forceinline__ void copy_chunk(unsigned char* dst, const ConvInput& in, int nx, int ny, int nz, int cin,
                                            int i, int j, int k, int c) {
-  const bool ok = i >= 0 && i < nx && j >= 0 && j < ny && k >= 0 && k < nz;
-  const __nv_bfloat16* src = in.x;
-  if (ok) {
-    if (c * 8 < in.ca)
-      src = in.coarse +
-            (((int64_t)(i >> 1) * ((ny + 1) >> 1) + (j >> 1)) * ((nz + 1) >> 1) + (k >> 1)) * in.ca + c * 8;
-    else
-      src = in.x + (((int64_t)i * ny + j) * nz + k) * (cin - in.ca) + (c * 8 - in.ca);
-  }
-  copy8<kVec>(dst, src, ok);
+  const bool ok = in_volume(nx, ny, nz, i, j, k);
+  copy8<kVec>(dst, ok ? channel_at(in, ny, nz, cin, i, j, k, c * 8) : in.x, ok);
 }
 
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
@@ -381,10 +385,35 @@ struct WgradTile {
   unsigned cols;
 };
 
+// One CTA's share of dw[co][tap (di, dj, dk)][ci], product by product.  The
+// row shifts of k_wgrad_tc pair zero rows of dy with voxels of x that are not
+// theirs (the halo columns of a box): nothing while x is finite, a NaN where it
+// is not.  A sum that came out infinite or NaN is formed again here.
+__device__ __noinline__ float wgrad_direct(const WgradArgs& A, const WgradTile& T, int di, int dj, int dk, int ci,
+                                           int co) {
+  float s = 0.0f;
+  for (int item = blockIdx.x; item < T.items; item += gridDim.x) {
+    const int z0 = (item % T.nzb) * T.bz, rest = item / T.nzb;
+    const int j0 = (rest % T.njb) * T.bj, i = rest / T.njb;
+    const int j1 = min(A.ny, j0 + T.bj), k1 = min(A.nz, z0 + T.bz);
+    for (int j = j0; j < j1; ++j)
+      for (int k = z0; k < k1; ++k) {
+        const float g = __bfloat162float(A.dy[(((int64_t)i * A.ny + j) * A.nz + k) * A.cout + co]);
+        float x = 0.0f;  // (times a dy that is infinite: NaN)
+        if (in_volume(A.nx, A.ny, A.nz, i + di, j + dj, k + dk))
+          x = __bfloat162float(*channel_at(A.in, A.ny, A.nz, A.cin, i + di, j + dj, k + dk, ci));
+        s = fmaf(g, x, s);
+        if (isnan(s)) return s;
+      }
+  }
+  return s;
+}
+
 // kVec: x and dy start on 16-byte boundaries (their rows are multiples of 32
 // bytes); they may start at any element otherwise.
 template <bool kVec>
-__global__ void __launch_bounds__(kThreads) k_wgrad_tc(WgradArgs A, WgradTile T) {
+__global__ void __launch_bounds__(kThreads) k_wgrad_tc(const __grid_constant__ WgradArgs A,
+                                                       const __grid_constant__ WgradTile T) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t tmem_slot;
@@ -476,9 +505,18 @@ __global__ void __launch_bounds__(kThreads) k_wgrad_tc(WgradArgs A, WgradTile T)
           float acc[16];
           tc_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((d * T.mb + m) * T.nt + c0), acc);
           if (di >= 3) continue;
+          unsigned again = 0;
 #pragma unroll
-          for (int q = 0; q < 16; ++q)
-            if (acc[q] != 0.0f) atomicAdd(A.dw + ((int64_t)(n0 + c0 + q) * 27 + t) * cin + ci, acc[q]);
+          for (int q = 0; q < 16; ++q) {
+            if (!isfinite(acc[q]))
+              again |= 1u << q;
+            else if (acc[q] != 0.0f)
+              atomicAdd(A.dw + ((int64_t)(n0 + c0 + q) * 27 + t) * cin + ci, acc[q]);
+          }
+          for (; again != 0; again &= again - 1) {
+            const int co = n0 + c0 + __ffs(again) - 1;
+            atomicAdd(A.dw + ((int64_t)co * 27 + t) * cin + ci, wgrad_direct(A, T, di - 1, dj, dk0 + d, ci, co));
+          }
         }
       }
   }

@@ -233,6 +233,30 @@ def test_weight_gradient_of_operands_at_any_element(x_off, g_off):
     assert _rel(dw.cpu().numpy(), _weight_gradient_reference(x, g, start).cpu().numpy()) <= 1e-5
 
 
+@pytest.mark.parametrize("shape", [(2, 3, 5), (3, 9, 130)])  # one box a plane, and lines split along z
+@pytest.mark.parametrize("where", ["x", "dy"])
+def test_weight_gradient_with_values_that_are_not_finite(shape, where):
+    """Infinities and a NaN on faces, a corner and a line's inside: each reaches
+    the taps that pair it with a voxel of the volume, and no other (in dy, zeros
+    outside the volume too: infinity times zero)."""
+    cin, cout = 16, 32
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(shape[2])
+    x, g = _volume(shape, cin, gen), _volume(shape, cout, gen)
+    bad = x if where == "x" else g
+    n = shape[2]
+    for (i, j, k), ch, value in (((0, 0, 0), 0, math.inf), ((shape[0] - 1, shape[1] - 1, n - 1), 1, -math.inf),
+                                 ((0, 1, n // 2), 2, math.inf), ((1, 0, n - 1), 3, math.nan), ((1, 2, 0), 4, math.inf),
+                                 ((1, 1, 1), 5, math.inf), ((1, 1, 2), 5, -math.inf)):
+        bad[i, j, k, ch] = value
+    dw = _weight_gradient(x, g, torch.zeros((cout, 27, cin), device="cuda")).double().cpu()
+    ref = _weight_gradient_reference(x, g, torch.zeros((cout, 27, cin), device="cuda")).cpu()
+    assert torch.equal(torch.isnan(dw), torch.isnan(ref))
+    assert torch.equal(torch.isinf(dw), torch.isinf(ref)) and torch.equal(dw[torch.isinf(dw)], ref[torch.isinf(ref)])
+    fin = torch.isfinite(ref)
+    assert not fin.all() and _rel(dw[fin].numpy(), ref[fin].numpy()) <= 1e-5
+
+
 # ---------------------------------------------------------------------------
 # single-CTA tail of the V-cycle
 # ---------------------------------------------------------------------------

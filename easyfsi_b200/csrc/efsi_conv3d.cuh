@@ -538,11 +538,15 @@ constexpr int kMaxSmem = 222 * 1024;
 inline int chunk_stride(int bytes) { return ((bytes + 127) & ~127) + 64; }
 
 // The CTAs of one SM together may not ask for more than its 512 tensor-memory
-// columns: the shared memory of a launch is raised until one more CTA than
-// they hold would not fit the SM.
+// columns, and convolutions and weight gradients (of several networks, too)
+// run beside each other: a launch takes the same share of the SM's 228 KB as
+// of its columns, less the 1 KB the system keeps per CTA and 256 bytes, so that
+// 512 / cols of them still fit.  The shares of all 512 columns leave at most
+// 4 KB, and the smallest CTA takes 14: whichever launches meet on an SM, their
+// columns fit it too.  (At the cap of kMaxSmem what is left holds no CTA.)
 inline int smem_for(int bytes, unsigned cols) {
-  const int n = 512 / (int)cols;
-  return std::max(bytes, 228 * 1024 / (n + 1) + 1024);
+  const int share = 228 * 1024 / 512 * (int)cols - 1024 - 256;
+  return std::max(bytes, std::min(share, kMaxSmem));
 }
 
 // The box of a convolution: among the line lengths, MMA tiles per plane,

@@ -328,6 +328,10 @@ __device__ __forceinline__ float div_by(float x, float w, float r) {
   return fabsf(e) <= 3.402823466e38f ? __fmaf_rn(e, r, q) : q;
 }
 
+// 1 / R for the tent; finite also for a radius so small that its reciprocal is
+// not, so that a particle at the marker itself keeps the quotient 0.
+__device__ __forceinline__ float tent_reciprocal(float R) { return fminf(__frcp_rn(R), 3.402823466e38f); }
+
 // hibm_mpm.py:4838-4848 tent weight.
 __device__ __forceinline__ float tent(const float* xm, const float* xp, float R, float rR) {
   float w = 1.0f;
@@ -439,7 +443,7 @@ __global__ void __launch_bounds__(32 * kMarkerWarps) k_scatter(BinView B, int M,
     const float xm[3] = {__ldg(xg + 3 * m), __ldg(xg + 3 * m + 1), __ldg(xg + 3 * m + 2)};
     const double Fm[3] = {__ldg(Fg + 3 * m), __ldg(Fg + 3 * m + 1), __ldg(Fg + 3 * m + 2)};
     const bool valid = finite3(xm) && isfinite(Fm[0]) && isfinite(Fm[1]) && isfinite(Fm[2]);
-    const float R = B.R, rR = __frcp_rn(R);
+    const float R = B.R, rR = tent_reciprocal(R);
     float wl = 0.0f;
     if (valid) for_near(B, xm, lane, [&](int p) { wl += tent(xm, xp + 3 * p, R, rR); });
     const float wsum = warp_allsum(wl);
@@ -489,7 +493,7 @@ __global__ void __launch_bounds__(32 * kMarkerWarps) k_feedback(BinView B, int M
     const float no[3] = {ng[3 * m], ng[3 * m + 1], ng[3 * m + 2]};
     const float ao = Ag[m];
     float vs[3] = {0, 0, 0}, ns[3] = {0, 0, 0}, as = 0.0f, ws = 0.0f, gs = 0.0f;
-    const float R = B.R, rR = __frcp_rn(R);
+    const float R = B.R, rR = tent_reciprocal(R);
     for_near(B, xo, lane, [&](int p) {
       float w = tent(xo, xp + 3 * p, R, rR);
       if (w > 0.0f) {

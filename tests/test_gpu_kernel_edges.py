@@ -368,6 +368,17 @@ def test_marker_exchange_ignores_particles_that_are_not_finite(count, radius):
     np.testing.assert_allclose(force[good], ref_force, rtol=0.0, atol=60 * 2.0**-24 * np.abs(marker_f).sum(0).max())
 
 
+def test_marker_exchange_with_a_radius_whose_reciprocal_overflows():
+    """A support radius of 1e-39 reaches the particle at the marker itself, with
+    weight one."""
+    origin = np.zeros((1, 3), np.float32)
+    force, state, scatter, feedback = _exchange(origin, np.ones((1, 3), np.float32), np.ones((1, 3), np.float32),
+                                                np.ones(1, np.float32), origin, np.array([[1.0, -2.0, 3.0]]), 1.0e-39)
+    assert scatter.active_marker_count == 1 and feedback.updated_marker_count == 1
+    np.testing.assert_array_equal(force, [[1.0, -2.0, 3.0]])
+    np.testing.assert_array_equal(state[1], [[1.0, 1.0, 1.0]])
+
+
 # ---------------------------------------------------------------------------
 # projection reports
 # ---------------------------------------------------------------------------

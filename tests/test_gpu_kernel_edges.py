@@ -289,6 +289,87 @@ def test_vcycle_tail_matches_the_oracle(nodes, outlet):
 
 
 # ---------------------------------------------------------------------------
+# column-marching kernels of the finest level
+# ---------------------------------------------------------------------------
+
+# odd nx (a last plane without its pair), ny % 8 != 0 and odd (partial tiles,
+# patches whose second row lies outside), nz on both sides of a 64-cell tile
+COLUMN_NODES = [(13, 9, 48), (5, 8, 64), (21, 19, 80), (8, 15, 144)]
+
+
+def _column_pair(nodes, rows, monkeypatch):
+    """The same problem with the column kernels and without them; with `rows`,
+    Dirichlet velocity rows weigh faces."""
+    from easyfsi_b200.fluid import CartesianFluidSolver, FluidDomainSpec
+
+    grid = _grid(nodes, True)
+    rng = np.random.default_rng(nodes[2])
+    obs = (rng.random(nodes) < 0.03).astype(np.int32)
+    act, weight = (rng.random(nodes) < 0.05).astype(np.int32), rng.random(nodes).astype(np.float32)
+    out = []
+    for off in (False, True):
+        with monkeypatch.context() as m:
+            if off:
+                m.setenv("EFSI_NO_COLUMN", "1")
+            else:
+                m.delenv("EFSI_NO_COLUMN", raising=False)
+            fl = CartesianFluidSolver(FluidDomainSpec((0, 0, 0), grid.bounds_max_m, None, 1000.0, 1.0e-3, 1.0e-3,
+                                                      cartesian_grid=grid))
+            fl.obstacle.from_numpy(obs)
+            if rows:
+                fl.velocity_dirichlet_boundary_active.from_numpy(act)
+                fl.velocity_dirichlet_boundary_projection_weight.from_numpy(weight)
+            fl._refresh_structure()
+        out.append(fl)
+    ofl = orc.OracleFluid(grid, rho=1000.0, mu=1.0e-3)
+    ofl.obstacle[...] = obs
+    return rng, obs, out, ofl
+
+
+@pytest.mark.parametrize("nodes", COLUMN_NODES)
+@pytest.mark.parametrize("rows", [False, True])
+@pytest.mark.parametrize("outlet", [0, 1])
+def test_column_vcycle_rows(nodes, rows, outlet, monkeypatch):
+    """A V-cycle without sums: bit for bit that of the other kernels, and the
+    oracle's (which takes no Dirichlet rows) to 1e-13 as in the general test."""
+    rng, obs, pair, ofl = _column_pair(nodes, rows, monkeypatch)
+    r = rng.normal(size=nodes) * (obs == 0)
+    z = []
+    for fl in pair:
+        fl.cg_r.from_numpy(r)
+        fl._apply_fv_multigrid_preconditioner(fl.cg_r, pressure_outlet_zmin=bool(outlet))
+        z.append(fl.cg_z.to_numpy())
+    np.testing.assert_array_equal(z[0], z[1])
+    if not rows:
+        assert _rel(z[0], ofl.vcycle(r, outlet)) <= 1e-13
+
+
+@pytest.mark.parametrize("nodes", COLUMN_NODES)
+@pytest.mark.parametrize("precond", ["fv_multigrid", "fv_multigrid_mixed"])
+@pytest.mark.parametrize("rows,outlet", [(False, 0), (False, 1), (True, 0), (True, 1)])
+def test_column_iterations(nodes, precond, rows, outlet, monkeypatch):
+    """Three CG iterations (a fresh direction, two with the last one added, the
+    dots in the last sweep): the rows are the same and only the order of the
+    f64 sums differs, 1e-11 of the pressure."""
+    rng, _, pair, ofl = _column_pair(nodes, rows, monkeypatch)
+    div = rng.normal(size=nodes).astype(np.float32)
+    p = []
+    for fl in pair:
+        fl.divergence.from_numpy(div)
+        fl.pressure.tensor.zero_()
+        fl._solve_pressure_poisson_fv_cg(iterations=3, rhs_scale=1.0e6, pressure_outlet_zmin=bool(outlet),
+                                         tolerance=1e-14, preconditioner=precond)
+        assert fl.last_cg_iterations == 3
+        p.append(fl.pressure.to_numpy())
+    assert _rel(p[0], p[1]) <= 1e-11
+    if precond == "fv_multigrid" and not rows and not outlet:
+        ofl.divergence[...] = div
+        ofl.prepare_rhs(1.0e6)
+        ofl.pcg_solve(outlet=0, max_iters=3, tol=1e-14, precond=1, remove_mean=True)
+        assert _rel(p[0], ofl.pressure) <= 1e-11
+
+
+# ---------------------------------------------------------------------------
 # particle binning
 # ---------------------------------------------------------------------------
 

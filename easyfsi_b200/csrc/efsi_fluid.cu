@@ -388,6 +388,11 @@ __device__ __forceinline__ void sample_tile(const LevelDev& L, const float* __re
   }
 }
 
+// Blocks per SM: three keep a point's state in registers; a single plane gets a
+// fourth (52 bytes of it spilled), which makes one wave of 592 blocks.
+template <int kNI>
+constexpr int kPredictBlocks = kNI == 1 ? 4 : 3;
+
 // fluid.py:2447-2513 _predict_kernel.  A block of 32 x 8 threads takes kNI
 // planes of a 32 (k) x 8 (j) column tile and first stages the previous
 // velocity of the tile and its one-cell halo in shared memory, one float4 per
@@ -401,8 +406,10 @@ __device__ __forceinline__ void sample_tile(const LevelDev& L, const float* __re
 // bytes a cell: 64 us at the copy rate), this takes 669 us: the issue slots of
 // the correctly rounded f32 arithmetic bound both.
 template <int kNI>
-__global__ void __launch_bounds__(kPK* kPJ, 3) k_predict(LevelDev L, efsi_grid_axes A, const float* __restrict__ vp,
-                                                      float dt, float nu, int rk2, float* __restrict__ vel) {
+__global__ void __launch_bounds__(kPK* kPJ, kPredictBlocks<kNI>) k_predict(LevelDev L, efsi_grid_axes A,
+                                                                           const float* __restrict__ vp, float dt,
+                                                                           float nu, int rk2,
+                                                                           float* __restrict__ vel) {
   extern __shared__ float4 ptile[];
   const int o0 = (int)blockIdx.z * kNI - 1, o1 = (int)blockIdx.y * kPJ - 1, o2 = (int)blockIdx.x * kPK - 1;
   for (int e = (int)(threadIdx.y * kPK + threadIdx.x); e < (kNI + 2) * kPH * kPW; e += kPK * kPJ) {
@@ -479,8 +486,7 @@ static void launch_predict(const LevelDev& L, const efsi_grid_axes& axes, const 
   const dim3 grid((unsigned)((L.nz + kPK - 1) / kPK), (unsigned)((L.ny + kPJ - 1) / kPJ),
                   (unsigned)((L.nx + kNI - 1) / kNI));
   constexpr size_t smem = sizeof(float4) * (kNI + 2) * kPH * kPW;
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(k_predict<kNI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static_assert(smem <= 48 * 1024, "what a launch gets without asking");
   EFSI_COUNTED k_predict<kNI><<<grid, dim3(kPK, kPJ), smem, s>>>(L, axes, vp, dt, nu, rk2, vel);
 }
 
@@ -807,13 +813,28 @@ int efsi_predict(efsi_fv_plan* P, const efsi_grid_axes* axes, const float* veloc
                  "predict needs distinct velocity and velocity_prev buffers");
   LevelDev L = level_dev(P, 0);
   cudaStream_t s = as_stream(stream);
-  // six planes a block (42 KB, three blocks per SM) read each tile 1.8 times
-  // over; two planes read it 2.7 times over but give a small grid three times
-  // the blocks, which is what counts until the SMs are full
-  const int64_t blocks6 = (int64_t)((L.nz + kPK - 1) / kPK) * ((L.ny + kPJ - 1) / kPJ) * ((L.nx + 5) / 6);
+  // Six planes a block read each tile 1.8 times over, two 2.7 times and one
+  // four times; fewer planes give a small grid more blocks, which counts until
+  // the SMs are full.  Times of a call with rk2 in us, with 1 / 2 / 6 planes a
+  // block (and one thread per cell without a tile):
+  //   12 x 12 x 16   8.6 / 12.4 / 24.7 (10.3)    72^3          31.8 / 34.0 / 32.8 (36.9)
+  //   48^3          12.4 / 14.4 / 24.6 (14.4)    80^3          37.7 / 37.0 / 32.9 (43.6)
+  //   56^3          18.5 / 15.2 / 24.7 (20.6)    96^3          51.5 / 49.7 / 55.5 (59.8)
+  //   64^3          20.6 / 24.7 / 28.4 (22.6)    112^3         86.6 / 86.1 / 81.7 (103)
+  //   64 x 64 x 96  26.7 / 26.7 / 28.8 (30.8)    160^3          228 / 220 / 190 (258)
+  //   45 x 61 x 143 30.8 / 29.7 / - (34.9)
+  // So: six from four blocks an SM on; one while that is a single wave, or
+  // while two planes leave a second wave nearly empty (up to 2.7 waves of one
+  // plane); two otherwise.
+  const int64_t tiles = (int64_t)((L.nz + kPK - 1) / kPK) * ((L.ny + kPJ - 1) / kPJ);
+  const int64_t blocks1 = tiles * L.nx, blocks2 = tiles * ((L.nx + 1) / 2), blocks6 = tiles * ((L.nx + 5) / 6);
+  const bool one = blocks1 <= 148 * kPredictBlocks<1> || (blocks2 > 148 * kPredictBlocks<2> && blocks1 < 1600);
   if (blocks6 >= 4 * 148)
     EFSI_TIMED(KF_PREDICT, 25.0 * P->lv[0].n, s,
                launch_predict<6>(L, *axes, velocity_prev, dt, nu, rk2, velocity, s));
+  else if (one)
+    EFSI_TIMED(KF_PREDICT, 25.0 * P->lv[0].n, s,
+               launch_predict<1>(L, *axes, velocity_prev, dt, nu, rk2, velocity, s));
   else
     EFSI_TIMED(KF_PREDICT, 25.0 * P->lv[0].n, s,
                launch_predict<2>(L, *axes, velocity_prev, dt, nu, rk2, velocity, s));

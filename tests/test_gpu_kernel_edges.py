@@ -111,7 +111,9 @@ def test_far_nodes_match_the_all_pairs_oracle(bands, slivers, triangles, nodes):
     ((4, 4, 4), False, 1.0e-2),
     ((9, 17, 33), True, 1.0e-2),    # one past a tile along j and k
     ((13, 8, 70), True, 2.0e-1),    # departure points several cells away
-    ((50, 65, 96), False, 1.0e-3),  # six planes a block
+    ((50, 65, 96), False, 1.0e-3),  # one plane a block, more than a wave
+    ((57, 45, 40), True, 1.0e-2),   # two planes a block, the last block with one
+    ((67, 123, 130), False, 1.0e-2),  # six planes a block, the last block with one
 ])
 @pytest.mark.parametrize("rk2", [False, True])
 def test_predictor_matches_the_oracle(nodes, graded, dt, rk2):

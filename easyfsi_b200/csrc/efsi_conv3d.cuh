@@ -162,7 +162,7 @@ struct ConvArgs {
 struct ConvTile {
   int bz, zp;        // output voxels per line, rows per line (bz + 2)
   int bj, bi;        // lines per plane, planes
-  int nt;            // output channels
+  int nt;            // output channels (the last split may have fewer)
   int mt;            // 128-row MMA tiles per plane
   int slots;         // planes in the ring: 3 (bi == 1) or 4
   int nzb, njb, nib; // boxes along z, y, x
@@ -259,7 +259,9 @@ __global__ void __launch_bounds__(kThreads) k_conv3d_tc(ConvArgs A, ConvTile T) 
   };
   for (int q = tid; q < 27 * nt * kch; q += kThreads) {
     const int c = q % kch, r = q / kch, t = r % 27, co = r / 27;
-    cp_async16(sw + ((t * kch + c) * nt + co) * 16, A.w + ((int64_t)(n0 + co) * 27 + t) * cin + c * 8, 16);
+    const bool in = n0 + co < A.cout;  // the last split may have fewer channels
+    cp_async16(sw + ((t * kch + c) * nt + co) * 16, in ? A.w + ((int64_t)(n0 + co) * 27 + t) * cin + c * 8 : A.w,
+               in ? 16 : 0);
   }
   for (int p = ib - 1; p <= ib + 1; ++p) load_plane(p);
   cp_async_commit();
@@ -294,7 +296,7 @@ __global__ void __launch_bounds__(kThreads) k_conv3d_tc(ConvArgs A, ConvTile T) 
       const int j = j0 + line, k = z0 + z - 1;
       const bool in = line < T.bj && z >= 1 && z <= T.bz && j < A.ny && k < A.nz;
       const int64_t at = (((int64_t)i * A.ny + j) * A.nz + k) * A.cout + n0;
-      for (int c0 = 0; c0 < nt; c0 += 16) {
+      for (int c0 = 0; c0 < min(nt, A.cout - n0); c0 += 16) {
         float acc[16];
         tc_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((buf * T.mt + m) * nt + c0), acc);
         if (!in) continue;
@@ -560,7 +562,8 @@ inline bool conv_tile(int nx, int ny, int nz, int cin, int cout, ConvTile& best)
   for (int zcap : {62, 30, 14, 6})
     for (int mt : {4, 2, 1})
       for (int nt = std::min(cout, 128) / 16 * 16; nt >= 16; nt -= 16) {
-        if (cout % nt != 0) continue;
+        const int splits = (cout + nt - 1) / nt;
+        if (nt > 16 && (cout + nt - 17) / (nt - 16) == splits) continue;  // 16 channels fewer do as well
         for (int bi : {16, 8, 4, 2, 1, 0}) {  // 0: one plane of one line, the least shared memory
           if (bi > 1 && bi > nx) continue;
           ConvTile t;
@@ -585,7 +588,7 @@ inline bool conv_tile(int nx, int ny, int nz, int cin, int cout, ConvTile& best)
           if (used > kMaxSmem || t.cols > 512) continue;
           t.smem = smem_for(used, t.cols);
           const int per_sm = std::max(1, 228 * 1024 / (t.smem + 1024));
-          const double ctas = (double)t.nzb * t.njb * t.nib * (cout / nt);
+          const double ctas = (double)t.nzb * t.njb * t.nib * splits;
           const double mma = (double)t.bi * mt * 27 * (kch / 2) * 36;
           const double copy = (w + (t.bi + 2.0) * rows * cin * 2) / 48;
           const double waves = std::max(1.0, std::ceil(ctas / (148.0 * per_sm)));

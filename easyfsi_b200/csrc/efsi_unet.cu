@@ -413,7 +413,7 @@ int conv_launch(const conv::ConvTile& T, const Dims& d, int cin, int cout, const
                 const float* bias, int relu, bf16* y, float* yf, int* error, cudaStream_t s) {
   conv::ConvArgs A{d.nx, d.ny, d.nz, cin, cout, in, w, bias, relu, y, yf, error};
   EFSI_TRY(set_kernel_attributes());
-  const dim3 grid((unsigned)(T.nzb * T.njb * T.nib), (unsigned)(cout / T.nt));
+  const dim3 grid((unsigned)(T.nzb * T.njb * T.nib), (unsigned)((cout + T.nt - 1) / T.nt));
   EFSI_COUNTED conv::k_conv3d_tc<<<grid, conv::kThreads, T.smem, s>>>(A, T);
   return EFSI_OK;
 }

@@ -157,7 +157,7 @@ def _shifted(x, t):
 CONV_SHAPES = [
     (16, 16, (1, 1, 1)), (16, 16, (2, 1, 62)), (16, 32, (3, 5, 63)), (48, 16, (17, 9, 65)), (16, 48, (5, 33, 130)),
     (64, 64, (4, 4, 4)), (112, 48, (3, 9, 34)), (48, 112, (2, 7, 16)), (176, 16, (3, 3, 64)), (64, 256, (2, 3, 5)),
-    (80, 32, (20, 18, 32)),
+    (80, 32, (20, 18, 32)), (48, 112, (16, 18, 32)),  # the last one: the last channel split has fewer
 ]
 
 

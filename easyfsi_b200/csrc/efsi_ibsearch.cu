@@ -140,8 +140,9 @@ struct SearchArgs {
   int nb[3];
   const int32_t* offset;   // null: every node visits every item
   const int32_t* entries;
-  const float4* rec;       // per item: kRecQuads quads (k_ibs_records)
+  const float4* rec;       // per item: kRecQuads quads (item_record)
   const float4* grp;       // per kGroup items: kGrpQuads quads (k_ibs_groups)
+  int far_here;            // few items: the search looks at all of them for a far node
   uint32_t* far_nodes;     // nodes left to k_ibs_far, and their count
   unsigned* far_count;
   // per-node fields (hibm_mpm.py:5418-5436) and the four report counts
@@ -186,7 +187,7 @@ __device__ __forceinline__ F3 oriented_normal(const SearchArgs& A, F3 fn, int ia
 }
 
 // Geometry of an item that no node changes, formed once per search by
-// k_ibs_records (a triangle's corners, its oriented unit normal; a marker's
+// item_record (a triangle's corners, its oriented unit normal; a marker's
 // position and normal), and what bounds its distances from below:
 //   q0 = (a, reach)   reach: the largest distance of the item's points from a
 //   q1 = (n, slack)   |s - dot(p - a, n)| <= slack + kSlackP |p|_1
@@ -198,9 +199,7 @@ constexpr float kSlack = 2.0e-5f;  // about 300 f32 units in the last place
 __device__ __forceinline__ F3 xyz(float4 q) { return f3(q.x, q.y, q.z); }
 __device__ __forceinline__ float abs1(F3 v) { return fabsf(v.x) + fabsf(v.y) + fabsf(v.z); }
 
-__global__ void k_ibs_records(SearchArgs A, float4* rec) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= items(A)) return;
+__device__ void item_record(const SearchArgs& A, int t, float4* rec) {
   float4* r = rec + (int64_t)kRecQuads * t;
   const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   r[2] = r[3] = zero;
@@ -416,9 +415,11 @@ __device__ __forceinline__ void item_bins(const SearchArgs& A, int t, int b0[3],
   }
 }
 
-__global__ void k_ibs_bin_count(SearchArgs A, int32_t* count, unsigned long long* total) {
+// The items' records and, per bin, how many items it lists.
+__global__ void k_ibs_bin_count(SearchArgs A, float4* rec, int32_t* count, unsigned long long* total) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= items(A)) return;
+  item_record(A, t, rec);
   int b0[3], b1[3];
   item_bins(A, t, b0, b1);
   if (b1[0] < b0[0]) return;
@@ -533,6 +534,15 @@ __device__ bool far_open(const SearchArgs& A, F3 p, float slack_p) {
   return true;
 }
 
+// Up to so many items a far node's thread looks at all of them itself: the
+// groups' bounds, the list of open nodes and k_ibs_far cost more than that.
+// A search in us, all items by the node's thread / open nodes by k_ibs_far:
+//   26 markers   16^3 101 / 128   96^3 157 / 329     48 triangles  16^3 271 / 299   96^3 1616 / 1817
+//   114 markers  16^3 132 / 146   96^3 243 / 406     120 triangles 16^3 264 / 254   96^3 1126 / 1240
+//   182 markers  16^3 157 / 151   96^3 307 / 416     224 triangles 16^3 301 / 242   96^3 1083 / 1024
+//   266 markers  16^3 182 / 154   96^3 384 / 441
+constexpr int kFewTriangles = 128, kFewMarkers = 192;
+
 // One thread per node (hibm_mpm.py:5837-6068 / 5603-5835).
 __global__ void __launch_bounds__(256) k_ibs_search(SearchArgs A) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -592,6 +602,26 @@ __global__ void __launch_bounds__(256) k_ibs_search(SearchArgs A) {
       kind = kNodeInternal;
       atomicAdd(A.report + 2, 1);
     }
+  } else if (A.far_here) {
+    Best global;
+    bool outside = false;
+    const int n = items(A);
+    for (int t = 0; t < n && !outside; ++t) {
+      if (__ldg(A.rec + (int64_t)kRecQuads * t).w < 0.0f) continue;  // degenerate
+      float d, s;
+      item_eval(A, t, p, d, s);
+      outside = s > A.tol;
+      global.offer(d, t);
+    }
+    if (!outside && global.t >= 0) {
+      kind = kNodeInternal;
+      F3 normal;
+      item_detail(A, global.t, p, marker, boundary, normal, ix, w);
+      float dsel;
+      item_eval(A, global.t, p, dsel, sd);
+      interior = add(boundary, scale(normal, A.probe));
+      atomicAdd(A.report + 2, 1);
+    }
   } else if (A.classify_far && far_open(A, p, slack_p)) {
     // the node may be internal: k_ibs_far looks at every item
     A.far_nodes[atomicAdd(A.far_count, 1u)] = (uint32_t)c;
@@ -607,7 +637,7 @@ __global__ void __launch_bounds__(256) k_ibs_search(SearchArgs A) {
   }
 }
 
-// The far nodes k_ibs_search left open (hibm_mpm.py:5937-6010: internal when no
+// The far nodes of a search with many items that k_ibs_search left open (hibm_mpm.py:5937-6010: internal when no
 // item at all sees the node outside, with the nearest of all items).  Items are
 // grouped by kGroup neighbours in index order (mesh order keeps them close to
 // each other), and a node asks a group's bounds (k_ibs_groups) before it asks
@@ -1337,7 +1367,9 @@ int efsi_ib_node_search(efsi_ib_search_plan* P, const efsi_ib_search_params* prm
   A.entries = nullptr;
   EFSI_TRY(grow(P->rec, P->rec_cap, (int64_t)kRecQuads * std::max(nitems, 1)));
   A.rec = P->rec;
-  if (A.classify_far) {
+  A.far_here = A.classify_far && nitems <= (prm->triangle_count > 0 ? kFewTriangles : kFewMarkers) ? 1 : 0;
+  const bool far_later = A.classify_far && !A.far_here;
+  if (far_later) {
     // 32-bit node indices: 2^32 nodes' fields would not fit the device
     EFSI_ARG_CHECK(A.n < (int64_t)1 << 32, "too many nodes");
     EFSI_TRY(grow(P->far_nodes, P->far_cap, A.n));
@@ -1346,13 +1378,6 @@ int efsi_ib_node_search(efsi_ib_search_plan* P, const efsi_ib_search_params* prm
     EFSI_CUDA_CHECK(cudaMemsetAsync(P->far_count, 0, sizeof(unsigned), s));
   }
   if (nitems > 0) {
-    EFSI_COUNTED k_ibs_records<<<(unsigned)((nitems + 255) / 256), 256, 0, s>>>(A, P->rec);
-    if (A.classify_far) {
-      const int ng = (nitems + kGroup - 1) / kGroup;
-      EFSI_TRY(grow(P->grp, P->grp_cap, (int64_t)kGrpQuads * ng));
-      A.grp = P->grp;
-      EFSI_COUNTED k_ibs_groups<<<(unsigned)((ng + 63) / 64), 64, 0, s>>>(A, P->grp);
-    }
     const int64_t tiles = (nbins + kScanTile - 1) / kScanTile;
     if (nbins > P->bin_cap) {
       cudaFree(P->count);
@@ -1372,7 +1397,13 @@ int efsi_ib_node_search(efsi_ib_search_plan* P, const efsi_ib_search_params* prm
     EFSI_CUDA_CHECK(cudaMemsetAsync(P->count, 0, (size_t)nbins * sizeof(int32_t), s));
     EFSI_CUDA_CHECK(cudaMemsetAsync(P->total, 0, sizeof(unsigned long long), s));
     const unsigned ig = (unsigned)((nitems + 255) / 256);
-    EFSI_COUNTED k_ibs_bin_count<<<ig, 256, 0, s>>>(A, P->count, P->total);
+    EFSI_COUNTED k_ibs_bin_count<<<ig, 256, 0, s>>>(A, P->rec, P->count, P->total);
+    if (far_later) {
+      const int ng = (nitems + kGroup - 1) / kGroup;
+      EFSI_TRY(grow(P->grp, P->grp_cap, (int64_t)kGrpQuads * ng));
+      A.grp = P->grp;
+      EFSI_COUNTED k_ibs_groups<<<(unsigned)((ng + 63) / 64), 64, 0, s>>>(A, P->grp);
+    }
     EFSI_LAUNCH_CHECK();
     EFSI_CUDA_CHECK(
         cudaMemcpyAsync(P->host_total, P->total, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
@@ -1391,7 +1422,7 @@ int efsi_ib_node_search(efsi_ib_search_plan* P, const efsi_ib_search_params* prm
     }
   }
   EFSI_COUNTED k_ibs_search<<<(unsigned)((A.n + 255) / 256), 256, 0, s>>>(A);
-  if (A.classify_far && nitems > 0) EFSI_COUNTED k_ibs_far<<<4 * 148, kFarWarps * 32, 0, s>>>(A);
+  if (far_later && nitems > 0) EFSI_COUNTED k_ibs_far<<<4 * 148, kFarWarps * 32, 0, s>>>(A);
   EFSI_LAUNCH_CHECK();
   return EFSI_OK;
 }

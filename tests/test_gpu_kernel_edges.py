@@ -66,7 +66,11 @@ def _closed_surface(bands, slivers):
 
 
 @pytest.mark.parametrize("bands,slivers,triangles,nodes", [
-    (3, False, True, (9, 11, 13)),     # fewer triangles than lanes and samples
+    (3, False, True, (9, 11, 13)),     # few triangles: looked at by the node's own thread
+    (4, True, True, (12, 10, 15)),     # ill-shaped and degenerate ones among them
+    (8, False, False, (13, 16, 11)),   # few markers
+    (5, True, True, (10, 9, 16)),      # a few more, on both sides of the line
+    (5, False, False, (10, 9, 16)),
     (6, True, True, (17, 9, 21)),      # one tile of items, ill-shaped triangles
     (12, False, False, (16, 16, 19)),  # markers without triangles
     (16, True, True, (20, 23, 31)),    # several tiles with a remainder

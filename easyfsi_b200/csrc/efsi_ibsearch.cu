@@ -220,6 +220,14 @@ __device__ void item_record(const SearchArgs& A, int t, float4* rec) {
   const F3 ab = sub(b, a), ac = sub(c, a), bc = sub(c, b);
   const float lab = norm(ab), lac = norm(ac), lbc = norm(bc);
   const float coords = kSlack * (abs1(a) + abs1(b) + abs1(c));
+  // The closest point closest_point gives lies in the triangle to a rounding of
+  // the coordinates, however far the node and however rounded d1 .. d6 are: on
+  // an edge its parameter is a quotient of a non-negative number by one at
+  // least as large, and inside va, vb and vc are the 2 x 2 determinants of
+  // (d1, d2), (d3, d4) and (d5, d6).  Any three such vectors satisfy
+  // va (d1, d2) + vb (d3, d4) + vc (d5, d6) = 0, from which the tests before
+  // have returned wherever one of the determinants is negative.  So the reach
+  // holds for short edges and distant nodes too.
   // In exact arithmetic p - closest and p - a have the same component along
   // the normal.  In f32 they differ by the rounding of the coordinates and by
   // how far the rounded edges leave the plane of the rounded normal.  A

@@ -106,6 +106,44 @@ def test_far_nodes_match_the_all_pairs_oracle(bands, slivers, triangles, nodes):
         np.testing.assert_allclose(got.to_numpy(), ref[key], rtol=0.0, atol=1e-6, err_msg=key)
 
 
+@pytest.mark.parametrize("edge", [2.0e-3, 5.0e-4, 1.0e-4])
+def test_far_nodes_of_a_fine_patch_match_the_all_pairs_oracle(edge):
+    """A patch of 1,152 irregular triangles with edges of a thousandth of the
+    nodes' distance and less, on a sphere that holds every node: each node is
+    internal, with the nearest of all triangles by the same f32 distances."""
+    from easyfsi_b200.hibm_mpm import HibmMpmIbNodeSearch, HibmMpmSurfaceMarkers
+
+    rng = np.random.default_rng(int(1.0 / edge))
+    m, nodes = 25, (7, 6, 9)
+    u, v = np.meshgrid(*[edge * (np.arange(m) - m / 2)] * 2, indexing="ij")
+    u, v = (q + 0.3 * edge * rng.uniform(-1.0, 1.0, (m, m)) for q in (u, v))
+    n = np.stack([u + 0.5, v + 0.3, np.full_like(u, 0.8)], axis=-1).reshape(-1, 3)
+    n /= np.linalg.norm(n, axis=1, keepdims=True)
+    x = (0.5 + 0.95 * n).astype(np.float32)
+    at = np.arange(m * m).reshape(m, m)
+    a, b, c, d = (q.ravel() for q in (at[:-1, :-1], at[1:, :-1], at[1:, 1:], at[:-1, 1:]))
+    tri = np.concatenate([np.stack([a, b, c], 1), np.stack([a, c, d], 1)]).astype(np.int32)
+    mk = HibmMpmSurfaceMarkers(marker_capacity=len(x), projection_triangle_capacity=len(tri))
+    mk.load_markers(positions_m=x.tolist(), velocities_mps=np.zeros_like(x).tolist(), normals=n.tolist(),
+                    areas_m2=[1.0] * len(x), region_ids=[1] * len(x))
+    mk.set_projection_triangles(tri.tolist())
+    search = HibmMpmIbNodeSearch(grid_nodes=nodes, bounds_min_m=(0.0, 0.0, 0.0), bounds_max_m=(1.0, 1.0, 1.0),
+                                 marker_capacity=len(x))
+    rep = search.search_and_classify(mk, search_radius_m=0.02, interior_probe_distance_m=0.02,
+                                     classify_far_internal_nodes=True)
+    ref = orc.ib_node_search(grid_nodes=nodes, markers_x=mk.x_gamma_m.to_numpy(), markers_n=mk.n_gamma.to_numpy(),
+                             triangles=tri, search_radius=0.02, interior_probe_distance=0.02,
+                             sign_tolerance=search._default_sign_tolerance_m(), classify_far=True,
+                             bounds_min=(0.0, 0.0, 0.0), spacing=search.spacing_m)
+    assert rep.__dict__ == ref["report"]
+    assert rep.internal_node_count == math.prod(nodes)
+    np.testing.assert_array_equal(search.nearest_marker.to_numpy(), ref["nearest_marker"])
+    np.testing.assert_array_equal(search.node_projection_marker_indices.to_numpy(), ref["projection_indices"])
+    for got, key in ((search.node_signed_distance_m, "signed_distance"), (search.node_boundary_point_m, "boundary_point"),
+                     (search.node_projection_marker_weights, "projection_weights")):
+        np.testing.assert_allclose(got.to_numpy(), ref[key], rtol=0.0, atol=1e-6, err_msg=key)
+
+
 # ---------------------------------------------------------------------------
 # predictor tiles
 # ---------------------------------------------------------------------------
@@ -381,27 +419,33 @@ def test_column_iterations(nodes, precond, rows, outlet, monkeypatch):
 
 
 @pytest.mark.parametrize("nodes", [(8, 8, 8), (80, 84, 76), (84, 84, 84)])
-def test_substep_over_many_tiles_conserves_mass_and_momentum(nodes):
-    """Tile counts on both sides of one scan block's 8192 entries: particles in
-    the first, middle and last tiles all reach the grid, so the reported mass
-    and momentum are the particles' (f32 products, f64 sums: 1e-6)."""
+def test_substep_over_many_tiles_matches_the_oracle(nodes):
+    """Tile counts on both sides of one scan block's 8192 entries, particles in
+    the first, middle and last tiles: the exchange with the grid changes every
+    particle's velocity, so one that a wrong offset leaves out of either transfer
+    keeps its own.  f32 sums by atomics in another order, 1e-5 as in the general
+    test; the report counts every particle."""
     from easyfsi_b200.neo_hookean_mpm import NeoHookeanMpmState
 
     rng = np.random.default_rng(nodes[1])
     lo, hi = 3.0 / np.asarray(nodes), 1.0 - 3.0 / np.asarray(nodes)
-    x = np.concatenate([lo + 0.02 * rng.random((40, 3)), 0.4 + 0.2 * rng.random((40, 3)), hi - 0.02 * rng.random((40, 3))])
-    v = rng.normal(size=x.shape).astype(np.float32) * 0.01
+    x = np.concatenate([lo + 0.02 * rng.random((40, 3)), 0.4 + 0.04 * rng.random((400, 3)),
+                        hi - 0.02 * rng.random((40, 3))]).astype(np.float32)
     n = len(x)
+    v = (0.01 * rng.normal(size=(n, 3))).astype(np.float32)
+    vol, mass = np.full(n, 1e-6, np.float32), np.full(n, 1e-3, np.float32)
     so = NeoHookeanMpmState(particle_capacity=n, bounds_min_m=(0, 0, 0), bounds_max_m=(1, 1, 1), grid_nodes=nodes)
-    so.load_particles(positions_m=x.astype(np.float32), volumes_m3=np.full(n, 1e-6, np.float32),
-                      masses_kg=np.full(n, 1e-3, np.float32), region_ids=np.full(n, 1, np.int32),
-                      normals=np.zeros((n, 3), np.float32), areas_m2=np.zeros(n, np.float32))
-    so.v.from_numpy(np.concatenate([v, np.zeros((so.v.tensor.shape[0] - n, 3), np.float32)]))
-    so.step(dt_s=1.0e-6, mu_pa=1.0e4, lambda_pa=1.0e4, primary_region_id=1, secondary_region_id=2,
-            velocity_damping=1.0, read_report=False)
-    got = so.v.to_numpy()[:n]
-    # nearly stress-free particles exchange momentum only with their neighbours
-    np.testing.assert_allclose(got.sum(0), v.sum(0), rtol=0.0, atol=1e-6 * np.abs(v).sum())
+    so.load_particles(positions_m=x, volumes_m3=vol, masses_kg=mass, region_ids=np.full(n, 1, np.int32))
+    so.v.tensor[:n] = torch.as_tensor(v, device=so.device)
+    ref = orc.OracleSolid(capacity=n, grid_nodes=nodes)
+    ref.load(x=x, volume=vol, mass=mass, region=np.full(n, 1, np.int32))
+    ref.v[:n] = v
+    rep = so.step(dt_s=1.0e-4, mu_pa=1.0e4, lambda_pa=1.0e4, primary_region_id=1, secondary_region_id=2)
+    ref.step(dt=1.0e-4, mu=1.0e4, lam=1.0e4, primary=1, secondary=2)
+    assert np.linalg.norm(ref.v[:n] - v, axis=1).min() > 1e-4  # every particle met the grid
+    for got, want in ((so.v, ref.v), (so.x, ref.x), (so.C, ref.C)):
+        assert _rel(got.to_numpy()[:n], want[:n]) <= 1e-5
+    assert rep.transfer_relative_error < 2e-5
 
 
 # ---------------------------------------------------------------------------
@@ -415,8 +459,9 @@ def _exchange(x, v, normal, area, marker_x, marker_f, radius):
 
     m = len(marker_x)
     mk = HibmMpmSurfaceMarkers(marker_capacity=m)
-    mk.load_markers(positions_m=marker_x.tolist(), velocities_mps=np.zeros_like(marker_x).tolist(),
+    mk.load_markers(positions_m=np.zeros((m, 3)).tolist(), velocities_mps=np.zeros_like(marker_x).tolist(),
                     normals=[(0.0, 0.0, 1.0)] * m, areas_m2=[1.0] * m, region_ids=[1] * m)
+    mk.x_gamma_m.from_numpy(marker_x)  # (loading refuses what is not finite)
     mk.F_gamma_n.from_numpy(marker_f)
     xt, vt, nt, at = (torch.from_numpy(q).cuda() for q in (x, v, normal, area))
     force = torch.zeros_like(xt)
@@ -453,6 +498,28 @@ def test_marker_exchange_ignores_particles_that_are_not_finite(count, radius):
         ref_scatter.active_marker_count, ref_scatter.invalid_marker_count, ref_scatter.active_particle_count)
     assert not force[bad].any()
     np.testing.assert_allclose(force[good], ref_force, rtol=0.0, atol=60 * 2.0**-24 * np.abs(marker_f).sum(0).max())
+
+
+def test_marker_exchange_with_markers_that_are_not_finite():
+    """Markers with a NaN or infinite position, or force, count as invalid and
+    leave the others' exchange as it is; a marker whose force alone is not finite
+    still moves with its particles."""
+    rng = np.random.default_rng(3)
+    x = rng.random((800, 3)).astype(np.float32)
+    v, normal = (rng.normal(size=(800, 3)).astype(np.float32) for _ in range(2))
+    area = rng.random(800).astype(np.float32)
+    marker_x, marker_f = x[:40].copy(), rng.normal(size=(40, 3))
+    bad_x, bad_f = np.array([0, 9, 39]), np.array([4, 17])
+    want = _exchange(x, v, normal, area, marker_x, np.where(np.isin(np.arange(40), bad_x)[:, None], 0.0, marker_f), 0.1)
+    marker_x[bad_x, [0, 1, 2]] = [np.nan, np.inf, -np.inf]
+    marker_f[bad_f, [0, 2]] = [np.nan, np.inf]
+    force, state, scatter, feedback = _exchange(x, v, normal, area, marker_x, marker_f, 0.1)
+    assert (scatter.active_marker_count, scatter.invalid_marker_count) == (35, 5)
+    assert (feedback.updated_marker_count, feedback.invalid_marker_count) == (37, 3)
+    assert np.isfinite(force).all() and math.isfinite(scatter.action_reaction_residual_n)
+    good = np.setdiff1d(np.arange(40), bad_x)
+    for got, ref in zip(state, want[1]):
+        np.testing.assert_array_equal(got[good], ref[good])
 
 
 def test_marker_exchange_with_a_radius_whose_reciprocal_overflows():
@@ -500,3 +567,60 @@ def test_dirichlet_row_report_sums(nodes):
     np.testing.assert_allclose(rep.momentum_delta_n_s, impulse, rtol=0.0,
                                atol=1e-6 * 1000.0 * h[0] * h[1] * h[2] * d.sum())
     np.testing.assert_array_equal(fl.velocity.to_numpy()[rows], val[rows])
+
+
+@pytest.mark.parametrize("nodes", [(4, 5, 6), (17, 9, 33), (40, 50, 60)])  # one block, some, more than a grid's turn
+@pytest.mark.parametrize("outlet", [0, 1])
+@pytest.mark.parametrize("value", [0.0, math.nan, math.inf])
+def test_final_divergence_report_slots(nodes, outlet, value):
+    """All nine categories against numpy: counts and maxima exact, sums of
+    squares to the order of f64 sums.  A value that is not finite stays in the
+    slots of its cell's categories."""
+    from ctypes import c_double
+
+    from easyfsi_b200 import _native
+    from easyfsi_b200.fluid import CartesianFluidSolver, FluidDomainSpec
+
+    grid = _grid(nodes, False)
+    fl = CartesianFluidSolver(FluidDomainSpec((0, 0, 0), grid.bounds_max_m, None, 1000.0, 1.0e-3, 1.0e-3,
+                                              cartesian_grid=grid))
+    rng = np.random.default_rng(nodes[0])
+    fluid = rng.random(nodes) > 0.3
+    act, reach = (rng.random(nodes) < 0.5).astype(np.int32), (rng.random(nodes) < 0.8).astype(np.int32)
+    div, src = (rng.normal(size=nodes).astype(np.float32) for _ in range(2))
+    iface = rng.normal(size=nodes)
+    cell = tuple(np.argwhere(fluid)[len(np.argwhere(fluid)) // 2])
+    if value != 0.0:
+        div[cell] = value
+    fl.obstacle.from_numpy((~fluid).astype(np.int32))
+    fl._refresh_structure()
+    gdiv, gsrc, gact, greach, giface = (torch.from_numpy(q).cuda() for q in (div, src, act, reach, iface))
+    out = (c_double * 54)()
+    _native.call("efsi_divergence_final_report", fl._plan, gdiv.data_ptr(), giface.data_ptr(), gsrc.data_ptr(),
+                 gact.data_ptr(), greach.data_ptr(), outlet, out, torch.cuda.current_stream().cuda_stream)
+    raw = np.abs(div.astype(np.float64) + iface)
+    res = np.abs(div.astype(np.float64) + iface - src)
+    va = act != 0
+
+    def ahead(m, axis):  # the next cell's value, False behind the last
+        return np.concatenate([np.delete(m, 0, axis), np.zeros_like(np.take(m, [0], axis))], axis)
+
+    def behind(m, axis):
+        return np.concatenate([np.zeros_like(np.take(m, [0], axis)), np.delete(m, -1, axis)], axis)
+
+    near, corr = va.copy(), np.zeros(nodes, bool)
+    for axis in range(3):
+        near |= ahead(va, axis)
+        corr |= (behind(fluid, axis) & ~va) | (ahead(fluid, axis) & ~ahead(va, axis))
+    if outlet:
+        corr[:, :, 0] |= ~va[:, :, 0]
+    inside = np.zeros(nodes, bool)
+    inside[1:-1, 1:-1, 1:-1] = True
+    on = fluid & (reach != 0)
+    sets = [on, on & inside, on & near, on & ~near, on & corr, on & ~corr, on & inside & corr, on & inside & ~corr,
+            fluid & (reach == 0)]
+    for q, cells in enumerate(sets):
+        for e, v in enumerate((raw[cells], res[cells])):
+            got = out[3 * (2 * q + e) : 3 * (2 * q + e) + 3]
+            assert got[2] == cells.sum()
+            np.testing.assert_allclose(got[:2], [v.max(initial=0.0), (v * v).sum()], rtol=1e-12, equal_nan=True)

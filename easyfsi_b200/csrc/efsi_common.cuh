@@ -92,6 +92,29 @@ void timing_end(int family, cudaStream_t s, double bytes);
 // launched without the attribute pdl_wait() returns at once.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// x / w with r = 1 / w rounded to nearest: the product x r, corrected by its
+// exact remainder (Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", 1990), rounds as the quotient does while nothing
+// underflows; a remainder that is not finite (x infinite or NaN, or the
+// quotient overflowing) leaves the product.  Three instructions and a select
+// instead of the full division, for divisors that a thread meets many times.
+__device__ __forceinline__ float div_by(float x, float w, float r) {
+  const float q = __fmul_rn(x, r);
+  const float e = __fmaf_rn(-q, w, x);
+  return fabsf(e) <= 3.402823466e38f ? __fmaf_rn(e, r, q) : q;
+}
+__device__ __forceinline__ double div_by(double x, double w, double r) {
+  const double q = __dmul_rn(x, r);
+  const double e = __fma_rn(-q, w, x);
+  return fabs(e) <= 1.7e308 ? __fma_rn(e, r, q) : q;
+}
+
+// The larger of two non-negative values by their bits, as an atomicMax of the
+// bits takes them: a NaN wins.
+__device__ __forceinline__ double max_nonneg(double a, double b) {
+  return (unsigned long long)__double_as_longlong(a) < (unsigned long long)__double_as_longlong(b) ? b : a;
+}
+
 // The V-cycle's kernels: after the wait a small grid lets the next kernel
 // launch, whose blocks then stand at their own wait (or form what the running
 // kernel cannot change, as the tail does) when this one ends.  The order of
@@ -99,8 +122,8 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // two blocks an SM does not: the waiting blocks would take the places of the
 // CG update's other half, which runs beside the V-cycle on its own stream
 // (128 x 128 x 256 coupled step 15.0 ms, 15.8 with every grid launching
-// early).  The CG's own kernels do not either: a Jacobi solve on 39 x 55 x 20
-// took 8.05 ms without and 8.31 with it.
+// early).  The CG's own kernels do not either: a Jacobi solve on 39 x 55 x 48
+// took 10.18 ms without and 10.56 with it.
 constexpr unsigned kEarlyLaunchBlocks = 2 * 148;
 __device__ __forceinline__ void pdl_wait_early() {
   pdl_wait();

@@ -160,11 +160,6 @@ __device__ __forceinline__ void atomic_max_nonneg(double* addr, double v) {
   atomicMax(reinterpret_cast<unsigned long long*>(addr), (unsigned long long)__double_as_longlong(v));
 }
 
-// The larger of two non-negative values by their bits: a NaN wins.
-__device__ __forceinline__ double max_nonneg(double a, double b) {
-  return (unsigned long long)__double_as_longlong(a) < (unsigned long long)__double_as_longlong(b) ? b : a;
-}
-
 // fluid.py:2549-2593 _apply_velocity_dirichlet_boundary_rows_kernel.  The
 // report's sums meet in the warp and the block before they go to memory: with
 // six atomics a row, all on one cache line, a shell of rows on 75 x 61 x 143
@@ -294,18 +289,6 @@ __device__ __forceinline__ void sample_prev(const LevelDev& L, const float* __re
     out[1] = fb[1];
     out[2] = fb[2];
   }
-}
-
-// x / w with r = 1 / w rounded to nearest: the product x r, corrected by its
-// exact remainder (Markstein, "Computation of elementary functions on the IBM
-// RISC System/6000 processor", 1990), rounds as the quotient does while
-// nothing underflows; a non-finite remainder (x infinite or NaN, or the
-// quotient overflowing) leaves the product.  Three instructions and a select
-// instead of the full division, for the divisors a thread meets many times.
-__device__ __forceinline__ float div_by(float x, float w, float r) {
-  const float q = __fmul_rn(x, r);
-  const float e = __fmaf_rn(-q, w, x);
-  return fabsf(e) <= 3.402823466e38f ? __fmaf_rn(e, r, q) : q;
 }
 
 // One axis around a cell: the centres of the cell and its two neighbours, the

@@ -851,16 +851,6 @@ __device__ void tail_build_tables(const TailDesc& T, int l, unsigned char* smem,
   }
 }
 
-// x / w with r = 1 / w rounded to nearest: the product corrected by its exact
-// remainder rounds as the quotient does while nothing underflows (Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000
-// processor", 1990); a remainder that is not finite leaves the product.
-__device__ __forceinline__ double tail_div(double x, double w, double r) {
-  const double q = x * r;
-  const double e = fma(-q, w, x);
-  return fabs(e) <= 1.7e308 ? fma(e, r, q) : q;
-}
-
 // Neighbour sum of row t from the tables (same order and fused multiply-adds
 // as `stencil`).
 __device__ __forceinline__ double tail_ns(const TailTables& tb, const float* p, int t) {
@@ -877,7 +867,7 @@ __device__ void tail_sweep(const TailTables& tb, const float* src, float* dst, c
     float res = 0.0f;
     if (rd != 0.0) {
       const double ns = src != nullptr ? tail_ns(tb, src, t) : 0.0;
-      const double jv = tail_div(ns - (double)rhs[t], tb.den[t], rd);
+      const double jv = div_by(ns - (double)rhs[t], tb.den[t], rd);
       const double pcur = src != nullptr ? (double)src[t] : 0.0;
       res = (float)(pcur + omega * (jv - pcur));
     }
@@ -915,7 +905,7 @@ __device__ int tail_sweeps_small(const TailTables& tb, float* const buf[2], int 
         for (int f = 1; f < 6; ++f) ns = fma(a[f], (double)src[nb[f]], ns);
       }
       const double pcur = (double)p;
-      const double jv = tail_div(ns - b, den, rd);
+      const double jv = div_by(ns - b, den, rd);
       p = rd != 0.0 ? (float)(pcur + omega * (jv - pcur)) : 0.0f;
       c = c < 0 ? 0 : 1 - c;
       if (t < tb.n) buf[c][t] = p;
@@ -2419,9 +2409,15 @@ int efsi_fv_plan_create(const efsi_level_desc* levels, int32_t n_levels, int32_t
       const MarchCfg ms = march_cfg(B.nx, B.ny, B.nz, nsm * 2);
       B.spchunk = ms.chunk;
       B.spgrid = ms.grid;
-      // the column kernels take two cells per thread along k: levels of at
-      // least 40 cells there fill most of a 64-cell tile (at 64^3 a coupled
-      // step takes the same time either way, at 128 x 128 x 256 13% less)
+      // The column kernels take two cells per thread along k; a 48-cell level
+      // is the narrowest that fills most of a 64-cell tile.  Microseconds per
+      // CG iteration with them / with the one-cell march:
+      //   nz 48: 32^2 71.3 / 70.0, 80^2 100.4 / 97.8, 96^2 102.6 / 112.6, 128^2 125.6 / 140.0
+      //   nz 64: 48^2 83.9 / 81.9, 64^2 89.4 / 90.3, 128^2 131.9 / 150.6
+      //   nz 80: 64^2 107.9 / 108.8, 128^2 183.4 / 183.4, 192^2 298.5 / 300.4
+      //   nz 96: 128^2 182.5 / 183.3    nz 112: 128^2 198 / 216    nz 144: 128^2 257 / 262
+      //   nz 256: 64^2 133.0 / 149.6, 128^2 303 / 356
+      // Small levels are within 2.5% either way, by how the chunks fall.
       B.column = l == 0 && B.march && B.nz >= 40 && std::getenv("EFSI_NO_COLUMN") == nullptr;
       const MarchCfg mc4 = column_cfg(B.nx, B.ny, B.nz, nsm * 4);
       B.cchunk = mc4.chunk;

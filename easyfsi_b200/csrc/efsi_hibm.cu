@@ -318,21 +318,12 @@ __global__ void k_bin_rank(int nbins, const int32_t* offset, const int32_t* in, 
   }
 }
 
-// x / w with r = 1 / w rounded to nearest: the product corrected by its exact
-// remainder rounds as the quotient does while nothing underflows (Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000
-// processor", 1990), and a quotient that does is lost beside the tent's 1.
-__device__ __forceinline__ float div_by(float x, float w, float r) {
-  const float q = __fmul_rn(x, r);
-  const float e = __fmaf_rn(-q, w, x);
-  return fabsf(e) <= 3.402823466e38f ? __fmaf_rn(e, r, q) : q;
-}
-
 // 1 / R for the tent; finite also for a radius so small that its reciprocal is
 // not, so that a particle at the marker itself keeps the quotient 0.
 __device__ __forceinline__ float tent_reciprocal(float R) { return fminf(__frcp_rn(R), 3.402823466e38f); }
 
-// hibm_mpm.py:4838-4848 tent weight.
+// hibm_mpm.py:4838-4848 tent weight.  (A quotient that underflows is lost beside
+// the tent's 1.)
 __device__ __forceinline__ float tent(const float* xm, const float* xp, float R, float rR) {
   float w = 1.0f;
 #pragma unroll
@@ -403,12 +394,6 @@ __device__ __forceinline__ double warp_allsum(double v) {
 // line took most of the exchange of 8,192 markers: the scatter took 87 us, the
 // feedback 59; with one report a block 53 and 47.
 constexpr int kMarkerWarps = 8;
-
-// The larger of two non-negative values by their bits, as atomic_max_nonneg_d
-// takes them: a NaN wins.
-__device__ __forceinline__ double max_nonneg(double a, double b) {
-  return (unsigned long long)__double_as_longlong(a) < (unsigned long long)__double_as_longlong(b) ? b : a;
-}
 
 // Adds (max_mask: keeps the larger of) the block's values; every thread takes part.
 template <int N>
@@ -564,7 +549,8 @@ __global__ void __launch_bounds__(32 * kMarkerWarps) k_feedback(BinView B, int M
   block_report(tot, 0xF0u, rep);
 }
 
-// A marker per warp in one wave; further markers in turn.
+// A marker per warp, up to eight blocks per SM; further markers in turn.  (64 and
+// 72 registers a thread: four and three blocks of them run at a time.)
 static unsigned marker_grid(int markers) {
   return (unsigned)std::max(1, std::min((markers + kMarkerWarps - 1) / kMarkerWarps, 8 * 148));
 }

@@ -257,7 +257,9 @@ __global__ void k_bin_keys(efsi_mpm_state S, int tx, int ty, int tz, int ntiles,
 // writes kScanTile consecutive entries and sums all the counts before them for
 // itself: the blocks need no order among each other, and what they read again
 // comes from L2, coalesced.  One block over everything, a run of counts per
-// thread, took 60.5 us of 117,649 tiles (196^3 nodes); this takes 7.3 us.
+// thread, took 60.5 us of 117,649 tiles (196^3 nodes); this takes 7.3 us.  (The
+// counts read again grow with the square of the tiles, a gigabyte at 500^3
+// nodes and 60 at 1000^3, where this is no faster than the one block.)
 // count, offset and cursor are cudaMalloc'd, so quads are aligned.
 constexpr int kScanPer = 8, kScanTile = 1024 * kScanPer;
 

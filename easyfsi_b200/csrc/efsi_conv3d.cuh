@@ -20,19 +20,22 @@
 // outside the volume) and write the previous plane's result: tcgen05.ld (warp
 // w owns lanes 32w..32w+31 = rows), bias, ReLU, BF16 (and optionally FP32).
 //
-// What bounds it: an MMA of N = 16..64 reads its 4 KB A operand from shared
-// memory in about 32 cycles, more than its tensor-core time, so the tensor
-// pipe cannot fill at these channel counts; the box is chosen (conv_tile) so
-// that enough CTAs run and few halo rows are computed.  With the voxels copied
-// again for every tap, a network forward at 64 x 72 x 128 took 1.89 ms; it takes
-// 1.14 ms now.
+// What bounds it: MMAs of N = 16..64 are short, and their rate is that of the
+// one thread that issues them and of the A operand's reads from shared memory
+// (4 KB, 32 cycles), so the tensor pipe cannot fill at these channel counts; the
+// box is chosen (conv_tile) so that enough CTAs run and few halo rows are
+// computed.  A network forward at 64 x 72 x 128 took 1.89 ms with the voxels
+// copied again for every tap, 1.14 ms without, and takes 0.84 ms now that the
+// issuing thread only adds to its descriptors (forming them anew took longer
+// than the MMAs: 80 -> 32 channels at 32^3 67.7 us, now 55.4; 16 -> 16 at 64 x 72
+// x 128 80.1, now 58.5).
 //
 // The weight gradient dW[co][t][ci] = sum_v dY[v][co] X[v + off(t)][ci] reads
 // the same images as MN-major operands (rows = voxels = K): A is the three
 // planes' chunks of X side by side, so M runs over (di, ci), N over co, and a
 // tap's (dj, dk) is again a row shift.
 // On the FP32 pipes it was 14.0 of the 18.2 ms of the gradients of four 32^3
-// crops; all of those take 5.1 ms now.
+// crops; all of those take 3.5 ms now.
 //
 // Every mbarrier wait is bounded; a wait that gives up sets the caller's
 // error word, waits (bounded) for the MMAs in flight and frees the tensor
@@ -270,20 +273,25 @@ __global__ void __launch_bounds__(kThreads) k_conv3d_tc(ConvArgs A, ConvTile T) 
   __syncthreads();
 
   const uint32_t idesc = idesc_bf16(kTileM, nt);
-  // the 27 taps of output plane i into accumulator set `buf`
+  // The 27 taps of output plane i into accumulator set `buf`.  A descriptor's
+  // low bits are the start address in 16-byte units, and a row is one: the
+  // thread that issues only adds to the two descriptors.
+  const uint64_t adesc = umma_desc(smem_u32(sx), (uint32_t)T.cs, 128);
+  const uint64_t bdesc = umma_desc(smem_u32(sw), (uint32_t)(nt * 16), 128);
   auto issue = [&](int i, int buf) {
     tc_fence_after();
     for (int m = 0; m < T.mt; ++m) {
       const uint32_t acc = tmem + (uint32_t)((buf * T.mt + m) * nt);
-      for (int t = 0; t < 27; ++t) {
-        const int di = t / 9 - 1, dj = (t / 3) % 3 - 1, dk = t % 3 - 1;
-        const uint32_t a0 = smem_u32(sx) + (uint32_t)(((i + di - ib + 1) % T.slots) * plane_bytes) +
-                            (uint32_t)((m * kTileM + (1 + dj) * zp + dk) * 16);
-        const uint32_t b0 = smem_u32(sw) + (uint32_t)(t * kch * nt * 16);
-        for (int ks = 0; ks < kch / 2; ++ks)
-          tc_mma(acc, umma_desc(a0 + (uint32_t)(2 * ks * T.cs), (uint32_t)T.cs, 128),
-                 umma_desc(b0 + (uint32_t)(2 * ks * nt * 16), (uint32_t)(nt * 16), 128), idesc,
-                 (t > 0 || ks > 0) ? 1 : 0);
+      uint64_t b = bdesc;
+      for (int di = 0; di < 3; ++di) {
+        // (dj, dk) of the plane i + di - 1: rows dj * zp + dk - 1 on
+        uint64_t plane = adesc + (uint64_t)(((i + di - ib) % T.slots) * rows + m * kTileM) - 1;
+        for (int dj = 0; dj < 3; ++dj, plane += zp)
+          for (int dk = 0; dk < 3; ++dk) {
+            uint64_t a = plane + dk;
+            for (int ks = 0; ks < kch / 2; ++ks, a += T.cs / 8, b += 2 * nt)
+              tc_mma(acc, a, b, idesc, (b != bdesc) ? 1 : 0);
+          }
       }
     }
     tc_commit(&bars[buf]);
@@ -556,12 +564,11 @@ inline int smem_for(int bytes, unsigned cols) {
 // cycles -- per SM, the CTAs it gets in turn, each a fixed start (about 4000
 // cycles: launch, first copies, first MMA) and 250 a plane, its copies at 64
 // bytes a cycle and its MMAs at 36 cycles (the A operand's shared-memory read).
-// The estimate ranks boxes, it does not time them (the measured times are 3.5
-// to 7 times as long).  Over 8408 boxes of 128 layer shapes, 2^3 to 64 x 72 x
-// 128 voxels and 16 to 112 channels, its choice is 1.4% off the best box on
-// average and 20% at worst; without the cycles per plane, which keep few CTAs
-// from marching over many planes, it was 5% and 92% (16 -> 16 channels at 48^3
-// 60.6 us, now 37.3; 48 -> 16 at 32^3 46.7, now 33.0).
+// The estimate ranks boxes, it does not time them (the measured times are 2.5
+// to 5 times as long).  Over 16530 boxes of 237 layer shapes, 2^3 to 96 x 96 x
+// 64 voxels and 16 to 112 channels, its choice is 2.3% off the best box on
+// average and 32% at worst; without the cycles per plane, which keep few CTAs
+// from marching over many planes, it is 5% and 82%.
 inline bool conv_tile(int nx, int ny, int nz, int cin, int cout, ConvTile& best) {
   double least = 1e300;
   const int kch = cin / 8;

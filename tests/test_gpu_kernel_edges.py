@@ -306,13 +306,16 @@ def test_weight_gradient_with_values_that_are_not_finite(shape, where):
 # ---------------------------------------------------------------------------
 
 
-@pytest.mark.parametrize("nodes,outlet", [
-    ((7, 6, 9), 0),      # two levels, 60 cells: two warps at the coarsest
-    ((8, 8, 8), 1),      # 64 + 8 cells, one warp
-    ((20, 17, 23), 0),   # 1080 cells: more than one a thread, odd extents
-    ((33, 17, 31), 1),   # 2448 + 360 + 60 cells: the first does not fit beside the others
+@pytest.mark.parametrize("nodes,outlet,solid", [
+    ((7, 6, 9), 0, 0.03),      # two levels, 60 cells: two warps at the coarsest
+    ((8, 8, 8), 1, 0.03),      # 64 + 8 cells, one warp
+    ((20, 17, 23), 0, 0.03),   # 1080 cells: more than one a thread, odd extents
+    ((33, 17, 31), 1, 0.03),   # 2448 + 360 + 60 cells: the first does not fit beside the others
+    ((16, 16, 16), 0, 0.15),   # the coarsest levels are obstacles throughout
+    ((16, 16, 16), 1, 0.6),    # all coarse levels are
+    ((20, 17, 23), 1, 0.0),
 ])
-def test_vcycle_tail_matches_the_oracle(nodes, outlet):
+def test_vcycle_tail_matches_the_oracle(nodes, outlet, solid):
     """The tail's rows round as the oracle's (quotients by a corrected
     reciprocal), so the V-cycle agrees to f64 rounding of the level-0 sweeps,
     1e-13 as in the general V-cycle test."""
@@ -323,7 +326,7 @@ def test_vcycle_tail_matches_the_oracle(nodes, outlet):
                                               cartesian_grid=grid))
     ofl = orc.OracleFluid(grid, rho=1000.0, mu=1.0e-3)
     rng = np.random.default_rng(nodes[0])
-    obs = (rng.random(nodes) < 0.03).astype(np.int32)
+    obs = (rng.random(nodes) < solid).astype(np.int32)
     fl.obstacle.from_numpy(obs)
     ofl.obstacle[...] = obs
     r = rng.normal(size=nodes) * (obs == 0)

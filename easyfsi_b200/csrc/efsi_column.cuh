@@ -26,13 +26,15 @@
 // coarse cell without leaving the thread, in the reference's order.
 //
 // What bounds them: the f64 row arithmetic and the division were issued at
-// 150 instructions a cell in the one-cell march (59% of the issue slots, DRAM
-// at 30%); here a row takes about a third of that and the kernels run closer
-// to the vectors' bytes.  On 128 x 128 x 256, one-cell march -> this, in us:
-// direction + SpMV 38.4 -> 28.4, sweep 28.6 -> 25.5, with the prolongation 44.5
-// -> 32.9, with the dots 44.4 -> 37.4, restriction 37.8 -> 25.7.  Every row is the same expression in the same order as
-// in `stencil`, so the results are bit for bit those of the other kernels;
-// only the order of the reductions follows the tile.
+// 130 instructions a cell in the one-cell march (59% of the issue slots, DRAM
+// at 30%).  Here it is 81; with 108 to 128 registers four blocks of four warps
+// run per SM, and the latency of the rows' f64 chains bounds them (issue slots
+// 35-48%, DRAM 27-48%).  On 128 x 128 x 256, one-cell march -> this, in us:
+// direction + SpMV 38.4 -> 29.3, sweep 28.6 -> 25.6, with the prolongation 44.5
+// -> 32.6, with the dots 44.4 -> 38.3, restriction 37.8 -> 25.8.  Every row is
+// the same expression in the same order as in `stencil`, so the results are bit
+// for bit those of the other kernels; only the order of the reductions follows
+// the tile.
 #pragma once
 
 #include "efsi_march.cuh"

@@ -509,8 +509,8 @@ int layer_backward(efsi_unet* U, const bf16* input, int l, const float* gy, floa
 // gradients run on the network's side stream: no later layer reads them, every
 // layer keeps its pre-activation gradient, and at small volumes neither they
 // nor the input gradients fill the GPU (the gradients of four 32^3 crops 5.1 ->
-// 3.9 ms, the sums of k_relu_back included).  Callers join
-// the side stream whatever is returned.
+// 3.9 ms with it and the sums of k_relu_back, before the convolutions' own
+// gains).  Callers join the side stream whatever is returned.
 int backward_layers(efsi_unet* U, const bf16* input, const float* dout, cudaStream_t s) {
   float* ga = U->w->gbuf[0];
   float* gb = U->w->gbuf[1];

@@ -64,8 +64,8 @@ int efsi_fv_kernel_replay(efsi_fv_plan* plan, int32_t family, int32_t reps, doub
  * the PCG's direction SpMV plus a whole V-cycle with the dots fused in; a
  * coarse level: its sweep + restriction -- under each candidate launch shape
  * (plane-marching kernels with 3, 1, 2, 4 or 6 blocks' worth of planes per
- * SM; on levels >= 1 also the tiled / per-cell kernels) and keeps the
- * fastest on the plan.  choice[l] is the blocks-per-SM multiple picked (0:
+ * SM, the column kernels of level 0 with 4, 2, 3, 6 or 8; on levels >= 1 also
+ * the tiled / per-cell kernels) and keeps the fastest on the plan.  choice[l] is the blocks-per-SM multiple picked (0:
  * tiled / per-cell kernels, -1: level not tuned) and best_us[l] the time of
  * its unit, for l < max_levels.  Needs the masks; drops the plan's captured PCG graphs
  * (the next solve records the tuned launches; a step graph captured before
